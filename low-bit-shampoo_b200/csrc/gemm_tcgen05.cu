@@ -286,7 +286,8 @@ template <int LEN>
 __device__ __forceinline__ void quantizing_epilogue(const CodeTables<16> &tab, const GemmParams &p, float (&sum)[LEN],
                                                     int b, int row, int n0, float alpha) {
     const bool lean_launch = !tab.lut_bad && !tab.need_clamp && tab.perm_identity && !tab.tiny_thr;
-    const float lut_scale = tab.lut_scale;
+    const int lut_shift = tab.lut_shift;
+    const unsigned lut_mask = tab.lut_mask;
 #pragma unroll
     for (int h = 0; h < LEN / 64; ++h) {
         const int c0 = n0 + h * 64;
@@ -336,33 +337,34 @@ __device__ __forceinline__ void quantizing_epilogue(const CodeTables<16> &tab, c
         const bool scale_ok = (amax >= 9.094947e-13f && amax <= 1.1529215e18f) || amax == 0.0f;
         const bool lean = lean_launch && scale_ok;
         unsigned char *cout = p.q_out + (long long)b * p.q_stride_codes + (e0 >> 1);
-        const float d = (amax == 0.0f) ? 1.0f : amax;
-        const float rcp = __frcp_rn(d);
+        const float rcp = __frcp_rz(amax == 0.0f ? 1.0f : amax);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
             if (g * 16 >= valid) continue;
             unsigned w0 = 0, w1 = 0;
-            if (lean) {
+            bool generic = !lean;
+            if (lean && amax != 0.0f) {                        // an all-zero block has codes 0 (functional.py:600-602)
+                unsigned w[16], nearest = 0xffffffffu;
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {
-                    const int i0 = lut_index(tab, tab.lut, lut_scale, div_by_recip(sum[h * 64 + g * 16 + j], d, rcp));
-                    const int i1 = lut_index(tab, tab.lut, lut_scale, div_by_recip(sum[h * 64 + g * 16 + j + 1], d, rcp));
-                    const unsigned byte = (unsigned)((i0 << 4) | i1);
-                    if (j < 8) w0 |= byte << (4 * j); else w1 |= byte << (4 * (j - 8));
+                for (int j = 0; j < 16; ++j) {
+                    w[j] = code_word(tab, lut_shift, lut_mask, sum[h * 64 + g * 16 + j], rcp);
+                    nearest = min(nearest, w[j] & 0xffffffu);
                 }
-                if (amax == 0.0f) { w0 = 0; w1 = 0; }          // functional.py:600-602
-            } else {
+                w0 = pack_codes(w);
+                w1 = pack_codes(w + 8);
+                generic = nearest <= 8u;
+            }
+            if (generic) {
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     LaneVals<8> xv;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) xv.v[j] = sum[h * 64 + g * 16 + q * 8 + j];
                     const unsigned long long pk = quantize_lane_generic<16, 8>(tab, xv, amax);
-                    unsigned w = 0;
+                    unsigned w[8];
 #pragma unroll
-                    for (int j = 0; j < 8; j += 2)
-                        w |= (unsigned)((((pk >> (8 * j)) & 15u) << 4) | ((pk >> (8 * (j + 1))) & 15u)) << (4 * j);
-                    if (q == 0) w0 = w; else w1 = w;
+                    for (int j = 0; j < 8; ++j) w[j] = (unsigned)(pk >> (8 * j)) << 24;
+                    (q == 0 ? w0 : w1) = pack_codes(w);
                 }
             }
             *reinterpret_cast<uint2 *>(cout + 8 * g) = make_uint2(w0, w1);

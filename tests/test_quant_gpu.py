@@ -121,6 +121,35 @@ def test_other_codebooks(F):
     check_against_oracle(F, A, uniform, 200, 64, 4, False)
 
 
+@pytest.mark.parametrize("bits,bs", [(4, 64), (4, 256), (8, 64), (8, 256), (8, 2048)])
+@pytest.mark.parametrize("n", [8, 9, 63, 65, 71, 129, 257, 263, 513, 1028])
+def test_rows_that_fit_no_vector_access(F, n, bits, bs):
+    """Orders whose rows start anywhere in an output word, last blocks of one to seven elements, both
+    dtypes and codebooks, values near the decision thresholds, zero and subnormal blocks, unaligned buffers."""
+    rng = np.random.default_rng(n * bits + bs)
+    code = qoracle.linear_map(True, bits, 2) if n % 2 else qoracle.dynamic_map(True, bits, 1)
+    mids = ((code[:-1].astype(np.float64) + code[1:]) / 2).astype(np.float32)
+    near = np.concatenate([mids, np.nextafter(mids, np.float32(2)), np.nextafter(mids, np.float32(-2)), [0.0, -0.0, 1e-30]]).astype(np.float32)
+    A = np.where(rng.random((n, n)) < 0.5, rng.choice(near, size=(n, n)), rng.standard_normal((n, n))).astype(np.float32)
+    A[:, ::bs] = 1.0
+    A[n // 3] = 0.0
+    A[n // 2] *= np.float32(1e-39)
+    for diagreal in (False, True):
+        check_against_oracle(F, A, code, n, bs, bits, diagreal)
+        A16 = torch.from_numpy(A).bfloat16().view(torch.int16).numpy().view(np.uint16)
+        check_against_oracle(F, A16, code, n, bs, bits, diagreal, in_bf16=True, out_bf16=True)
+    # buffers that start on no vector boundary
+    dev, dcode = "cuda:0", torch.from_numpy(code).to("cuda:0")
+    a = torch.empty(n * n + 1, device=dev)[1:].copy_(torch.from_numpy(A).reshape(-1)).view(n, n)
+    out = torch.zeros((n * n * bits + 7) // 8 + 1, dtype=torch.uint8, device=dev)[1:]
+    q, am = F.quantize_blockwise(a, dcode, n, out=out, blocksize=bs, bits=bits)
+    d = torch.empty(n * n + 1, device=dev)[1:].view(n, n)
+    F.dequantize_blockwise(q, dcode, n, am, out=d, blocksize=bs, bits=bits)
+    ref = qoracle.quantize(A, code, n, bs, bits, store_diag=False)
+    assert bits_equal(q.cpu().numpy(), ref[0]) and bits_equal(am.cpu().numpy(), ref[1])
+    assert bits_equal(d.cpu().numpy(), qoracle.dequantize(ref[0], code, n, ref[1], bs, bits))
+
+
 def test_near_threshold_values(F):
     """Inputs placed within a few ulps of every decision threshold of the codebook."""
     code = qoracle.linear_map(True, 4, 2)
