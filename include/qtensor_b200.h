@@ -487,6 +487,37 @@ int qt_adamw_tail(const long long *p_ptrs, const long long *d_ptrs, const long l
 int qt_column_dot(const float *A, const float *B, long long ld, long long stride, int rows, int cols, int batch,
                   float *out, long long stride_out, void *stream);
 
+/*
+ * The recurring part of an optimizer step - preconditioned directions of all gradient blocks, norm grafting, AdamW or
+ * SGD tail (optimizers/shampoo2.py:234-272, :441-466) - as five launches over tables that the caller lays out once
+ * (optimizers/_apply.py documents and fills them).  Additive.
+ *   items    80-byte work items (type, parameter, sizes, addresses);
+ *   groups   blocks of one shape, QT_APPLY_GROUP_BYTES each, filled in HOST memory by qt_apply_group() and then copied
+ *            to the device (128-byte aligned); at most 256 per wave;
+ *   tiles    first tile of every group and the total (n_groups + 1 ints);
+ *   waves    slices of the blocks that share one plane workspace.
+ * `grads` is a device array of the gradients' addresses, the only table that changes from step to step.
+ * kind 0: AdamW with factors s0, s1, s2 = 1/sqrt(1-beta2^t), -lr/(1-beta1^t), 1 - lr*weight_decay (from `scalars` in
+ * device memory if not NULL); kind 1: SGD with momentum.
+ */
+#define QT_APPLY_GROUP_BYTES 640
+typedef struct qt_apply_wave {
+    const void *plane_items; const void *groups1, *groups2; const int *tiles1, *tiles2;
+    int n_plane_items, n_groups, n_tiles1, n_tiles2, bn, reserved;
+} qt_apply_wave;
+typedef struct qt_apply_desc {
+    const void *stat_items; const qt_apply_wave *waves; const long long *grads; const float *code;
+    float *part_amax, *part_ss; int *pexp, *gexp;
+    const void *tensors; const int *chunk_tensor, *chunk_index; const void *ranges; const float *scalars;
+    int n_stat_items, n_waves, target, n_chunks, chunk_elems, kind, nesterov, reserved;
+    float s0, s1, s2, beta1, beta2, a1, a2, eps, lr, momentum, weight_decay;
+} qt_apply_desc;
+int qt_apply_group(void *out, const void *Ahi, const void *Alo, long long lda, long long strideA, const void *Bhi, const void *Blo,
+                   long long ldb, long long strideB, int M, int N, int K, int batch, int bn, int tile0,
+                   const int *a_exp, const int *b_exp, void *Phi, void *Plo, long long ldp, long long strideP, int *out_exp, int rel,
+                   void *D, long long ldd, int wide, float *part);
+int qt_apply_run(const qt_apply_desc *desc, void *stream);
+
 /* Sticky device-side error word (QT_OK or QT_ERR_TIMEOUT); synchronises the device.
  * clear != 0 resets it.  Additive; the reference has no device-side waits. */
 int qt_device_error(int clear);

@@ -50,6 +50,7 @@ struct DequantArgs {
     void *out; int out_dtype; long long stride_out;         // elements
 };
 
+int read_apply_error(bool clear);  // error word of the kernels in apply_kernels.cu
 int launch_merge_t(const float *G, long long ldg, long long strideG, const float *Tp, long long strideTp, int wo, int count,
                    float *T, long long strideT, cudaStream_t stream);
 int launch_quantize(const QuantArgs &a, cudaStream_t stream);

@@ -17,9 +17,11 @@ import torch.optim as optim
 
 import qtensor.functional as F
 from qtensor.utils import QTensorDiagReal, QTensorSVDFast
+from optimizers import _apply
 from optimizers import _engine as E
 
 FUSED_TAIL = True              # AdamW tail as one multi-tensor launch of the library (CUDA fp32 parameters)
+PLANNED_APPLY = True           # directions, grafting and tail of an unsharded step through a plan (optimizers/_apply.py)
 
 CODE = 'linear-2'
 
@@ -286,6 +288,7 @@ class _ShampooBase(optim.Optimizer):
         self._plans = {}
         self._use_graph = False
         self._graph_state = None
+        self._apply_plans = {}
         if process_group is not None:
             import torch.distributed as dist
             self._world = dist.get_world_size(process_group)
@@ -352,6 +355,7 @@ class _ShampooBase(optim.Optimizer):
         # captured graphs, pointer tables and exchange plans refer to the state that was just replaced
         self._graph_state = None
         self._plans = {}
+        self._apply_plans = {}
         for name in ("_tail_cache", "_scalar_ring", "_tail_scalars", "_pending_exchange", "_stable_direction_ptrs", "_last_tail_tab"):
             self.__dict__.pop(name, None)
         self._needs_eager = True                           # the next step rebuilds them eagerly
@@ -420,32 +424,101 @@ class _ShampooBase(optim.Optimizer):
         """Persistent buffers the update directions should be produced in, by parameter index (none here)."""
         return {}
 
-    def _precondition(self, group, params, split_exchange=False):
-        """Runs the statistics / inverse-root / apply phases for `params` (all with grads) and
-        returns the list of update directions (grafted to the gradient norm where active).
-        With `split_exchange` the sharded exchange stops after the pack: the caller then calls
-        _exchange_collective() and _exchange_unpack() itself."""
-        self._pending_exchange = None
+    def _refresh(self, group, params):
+        """Counts the step and refreshes statistics and inverse roots of `params` where their intervals fire."""
         t1, t2 = group['stat_compute_steps'], group['prec_compute_steps']
-        start = group['start_prec_step']
-        stat_items, root_items, apply_list = [], [], []
+        stat_items, root_items = [], []
         w1 = group['stat_decay']
         w2 = 1.0 if w1 == 1.0 else 1.0 - w1
         for p in params:
             state = self.state[p]
             state['step'] += 1
-            pre = state['preconditioner']
-            if state['step'] % t1 == 0 and pre.statistics:
-                stat_items += pre.statistics_items(p.grad.data)
-        for p in params:
-            state = self.state[p]
-            pre = state['preconditioner']
+            if state['step'] % t1 == 0:
+                pre = state['preconditioner']
+                if pre.statistics:
+                    stat_items += pre.statistics_items(p.grad.data)
             if state['step'] % t2 == 0:
+                pre = state['preconditioner']
                 root_items += pre._slots
                 pre._active = True
         if stat_items or root_items:
             E.refresh(stat_items, root_items, w1, w2, group['matrix_eps'], group.get('inv_root_mode', 0),
                       exact=(group.get('inv_root_mode', 0) != 0))
+
+    # ---- planned application (optimizers/_apply.py) ------------------------------------------
+    _plan_kind, _plan_moments = None, ()                      # set by the SGD / AdamW variants
+
+    def _plan_for(self, group, params, step):
+        """The plan for these parameters at this step, or None where the general path has to take it: sharded or
+        CPU runs, 16/32-bit preconditioners, gradients that are not dense fp32, steps that differ between parameters."""
+        if (not PLANNED_APPLY or self._plan_kind is None or self._world > 1 or F.lib is None or E.REFERENCE_DIAGREAL_NONE
+                or not E.USE_TENSOR_CORES or group['prec_bits'] not in (4, 8) or not FUSED_TAIL):
+            return None
+        ids = tuple(map(id, params))
+        known = self._apply_plans.get(ids)
+        if known is None:
+            if len(self._apply_plans) >= 4:                   # bounded: plans own workspaces
+                self._apply_plans.clear()
+            known = self._apply_plans[ids] = {"params": params, "states": [self.state[p] for p in params], "plans": {}}
+        states = known["states"]
+        for st in states:
+            if st['step'] != step:
+                return None
+        grafted = tuple([st['preconditioner']._active for st in states]) if step >= group['start_prec_step'] else (False,) * len(states)
+        plan = known["plans"].get(grafted)
+        if plan is None:
+            dev = params[0].device
+            if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
+                return None
+            if dev.type != "cuda" or any(p.device != dev or p.dtype != torch.float32 for p in params):
+                plan = False
+            else:
+                if len(known["plans"]) >= 2:
+                    known["plans"].clear()
+                with torch.cuda.device(dev):
+                    plan = _apply.ApplyPlan(params, states, grafted, self._plan_kind, self._plan_moments)
+                if not plan.ok:
+                    plan = False
+            known["plans"][grafted] = plan
+        if plan is False or not plan.bind_state():
+            return None
+        return plan
+
+    def _apply_planned(self, group, params, scalars=None):
+        """Directions, grafting and tail through the plan; False (nothing done) if there is none for this step.
+        The step has been counted already."""
+        step = self.state[params[0]]['step']
+        plan = self._plan_for(group, params, step)
+        if plan is None:
+            return False
+        table = self.__dict__.get("_grad_table")              # a captured step reads its own gradient buffers
+        if table is None:
+            ptrs = []
+            for p in params:
+                g = p.grad
+                if g.dtype != torch.float32 or not g.is_contiguous():
+                    return False
+                ptrs.append(g.data_ptr())
+            if torch.cuda.is_current_stream_capturing() and ptrs != plan.grads.ptrs:
+                return False
+            plan.grads.set(ptrs)
+            table = plan.grads.dev
+        with F._on_device(table):
+            plan.run(table, F._stream(table), scalars, **self._plan_hyper(group, step))
+        return True
+
+    def _precondition(self, group, params, split_exchange=False):
+        """Runs the statistics / inverse-root / apply phases for `params` (all with grads) and
+        returns the list of update directions (grafted to the gradient norm where active).
+        With `split_exchange` the sharded exchange stops after the pack: the caller then calls
+        _exchange_collective() and _exchange_unpack() itself."""
+        self._refresh(group, params)
+        return self._directions(group, params, split_exchange)
+
+    def _directions(self, group, params, split_exchange=False):
+        self._pending_exchange = None
+        start = group['start_prec_step']
+        apply_list = []
         directions = []
         for p in params:
             state = self.state[p]
@@ -537,9 +610,22 @@ class _ShampooBase(optim.Optimizer):
             fresh = any(len(self.state[p]) == 0 for p in params) or self.__dict__.get("_needs_eager", False)
             self._create_states(group, params)
             if self._use_graph and not fresh and self._graph_eligible(group, params):
+                step = self.state[params[0]]['step'] + 1
+                if step % group['stat_compute_steps'] and step % group['prec_compute_steps'] and self._plan_step(group, params):
+                    continue                                  # nothing fires: five launches need no graph
                 self._graph_step(group, params)
             else:
                 self._apply_update(group, params)
+
+    def _plan_step(self, group, params):
+        """A whole step in which no interval fires, or False (nothing done)."""
+        for p in params:
+            self.state[p]['step'] += 1
+        if self._apply_planned(group, params):
+            return True
+        for p in params:
+            self.state[p]['step'] -= 1
+        return False
 
     # ---- optional CUDA-graph execution of the step --------------------------------------
     def enable_cuda_graph(self, on=True):
@@ -565,6 +651,18 @@ class _ShampooBase(optim.Optimizer):
             return False
         return len({self.state[p]['step'] for p in params}) == 1
 
+    def _prepare_plan(self, group, params, step, fires_root):
+        """Builds the plan that a step about to be captured will look up (nothing may be uploaded during a capture)."""
+        states = [self.state[p] for p in params]
+        book = [(st['step'], st['preconditioner']._active) for st in states]
+        for st in states:
+            st['step'] = step
+            if fires_root:
+                st['preconditioner']._active = True
+        self._plan_for(group, params, step)
+        for st, (n, act) in zip(states, book):
+            st['step'], st['preconditioner']._active = n, act
+
     def _graph_step(self, group, params):
         gs = self._graph_state
         ids = tuple(id(p) for p in params)
@@ -574,6 +672,7 @@ class _ShampooBase(optim.Optimizer):
                 "grads": [torch.empty_like(p.grad) for p in params],
                 "scalars": torch.zeros(3, device=params[0].device),
             }
+            gs["table"] = torch.tensor([g.data_ptr() for g in gs["grads"]], dtype=torch.int64).to(params[0].device)
         step = self.state[params[0]]['step'] + 1
         fires_stat = step % group['stat_compute_steps'] == 0
         fires_root = step % group['prec_compute_steps'] == 0
@@ -602,8 +701,11 @@ class _ShampooBase(optim.Optimizer):
                 first_half_ran = False
                 try:
                     if self._world == 1:
+                        self._prepare_plan(group, params, step, fires_root)
+                        self._grad_table = gs["table"]
                         with torch.cuda.graph(graph):
                             self._apply_update(group, params, scalars=gs["scalars"])
+                        self._grad_table = None
                     else:
                         # sharded: graph 1 ends with this rank's directions packed into the send buffer,
                         # the all-gather runs eagerly, graph 2 unpacks and applies the tail
@@ -618,6 +720,7 @@ class _ShampooBase(optim.Optimizer):
                             self._exchange_unpack(params, directions)
                             self._apply_tail(group, params, directions, scalars=gs["scalars"])
                 except Exception as exc:
+                    self._grad_table = None
                     warnings.warn(f"CUDA-graph capture of the optimizer step failed ({exc!r}); running eagerly")
                     if first_half_ran:                          # statistics, roots and the exchange are done: finish the step
                         self._use_graph = False
@@ -676,8 +779,16 @@ class ShampooSGDBase(_ShampooBase):
     def _init_moments(self, p, state):
         state['momentum'] = torch.zeros_like(p, memory_format=torch.preserve_format)
 
+    _plan_kind, _plan_moments = 1, ('momentum',)
+
+    def _plan_hyper(self, group, step):
+        return dict(lr=group['lr'], momentum=group['momentum'], weight_decay=group['weight_decay'], nesterov=int(group['nesterov']))
+
     def _apply_update(self, group, params):
-        directions = self._precondition(group, params)
+        self._refresh(group, params)
+        if self._apply_planned(group, params):
+            return
+        directions = self._directions(group, params)
         wd, mom = group['weight_decay'], group['momentum']
         for p, d in zip(params, directions):
             buf = self.state[p]['momentum']
@@ -809,9 +920,19 @@ class ShampooAdamWBase(_ShampooBase):
                                      1.0 - float(beta1), 1.0 - float(beta2), float(group['eps']), F._stream(params[0]))
         F._check(rc, "adamw tail")
 
+    _plan_kind, _plan_moments = 0, ('exp_avg', 'exp_avg_sq')
+
+    def _plan_hyper(self, group, step):
+        beta1, beta2 = group['betas']
+        s = [0.0, 0.0, 0.0]
+        self._graph_scalars(group, step, s)
+        return dict(s0=s[0], s1=s[1], s2=s[2], beta1=beta1, beta2=beta2, a1=1.0 - beta1, a2=1.0 - beta2, eps=group['eps'])
+
     def _apply_update(self, group, params, scalars=None):
-        directions = self._precondition(group, params)
-        self._apply_tail(group, params, directions, scalars)
+        self._refresh(group, params)
+        if self._apply_planned(group, params, scalars):
+            return
+        self._apply_tail(group, params, self._directions(group, params), scalars)
 
     def _apply_tail(self, group, params, directions, scalars=None):
         if self._fused_tail_ok(params, directions):

@@ -1,0 +1,72 @@
+"""The planned application of the preconditioners (tables, grouped products, fused tail) against the general path of
+the same optimizer on the same state: ragged and small orders, split parameters, blocks with one plain fp32
+preconditioner, parameters without any, both tails, both code widths."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def run(kind, shapes, planned, bits=4, steps=3, wave_bytes=None, **hyper):
+    from optimizers import _apply, _base, shampoo2
+    g = torch.Generator(device="cuda").manual_seed(3)
+    ps = [torch.nn.Parameter(torch.randn(s, generator=g, device="cuda") * 0.1) for s in shapes]
+    cls = shampoo2.ShampooAdamW if kind == "adamw" else shampoo2.ShampooSGD
+    opt = cls(ps, lr=1e-2, weight_decay=0.03, prec_maxorder=200, prec_bits=bits, stat_compute_steps=10 ** 9, prec_compute_steps=1, **hyper)
+    before = _base.PLANNED_APPLY, _apply.WAVE_BYTES
+    _base.PLANNED_APPLY = planned
+    if wave_bytes:
+        _apply.WAVE_BYTES = wave_bytes
+    try:
+        for k in range(steps):
+            for p in ps:
+                p.grad = torch.randn(p.shape, generator=g, device="cuda") * 10.0 ** (k - 2)
+            opt.step()
+            if k == 0:                                   # dense preconditioners from here on
+                opt.param_groups[0]["prec_compute_steps"] = 10 ** 9
+                for p in ps:
+                    for q in opt.state[p]["preconditioner"].preconditioners:
+                        n = q.var.shape[0] if q.bits >= 16 else q.var_order
+                        a = torch.randn(n, n, generator=g, device="cuda") / n ** 0.5
+                        q.quantize(torch.eye(n, device="cuda") + 0.3 * (a + a.T))
+        assert bool(opt._apply_plans) == planned
+        assert all(pl for known in opt._apply_plans.values() for pl in known["plans"].values())
+    finally:
+        _base.PLANNED_APPLY, _apply.WAVE_BYTES = before
+    names = ("exp_avg", "exp_avg_sq") if kind == "adamw" else ("momentum",)
+    return [p.detach() for p in ps] + [opt.state[p][n] for n in names for p in ps] + [p.grad for p in ps if p.dim() < 2]
+
+
+SHAPES = [(64, 64), (65, 129), (200, 72), (7,), (300, 450), (200, 200, 1, 1), (5, 96), (96, 3, 3, 3), (1, 130, 77), (128, 199), (64, 64), (1,)]
+
+
+@pytest.mark.parametrize("kind,bits,hyper", [("adamw", 4, {}), ("adamw", 8, {}), ("sgd", 4, {}), ("sgd", 4, dict(nesterov=True, momentum=0.5)),
+                                             ("adamw", 4, dict(start_prec_step=3))])
+def test_planned_application_matches_the_general_path(kind, bits, hyper, native_lib):
+    a = run(kind, SHAPES, True, bits, **hyper)
+    b = run(kind, SHAPES, False, bits, **hyper)
+    for x, y in zip(a, b):
+        assert float((x - y).norm()) <= 3e-6 * float(y.norm()) + 1e-12
+    assert native_lib.qt_device_error(1) == 0
+
+
+def test_waves_give_the_same_bits(native_lib):
+    a, b = run("adamw", SHAPES, True), run("adamw", SHAPES, True, wave_bytes=1 << 19)
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+def test_gradients_that_move_and_graph_replay(native_lib):
+    """Gradients at new addresses every step (above) and steps under cuda_graph=True give the eager results."""
+    a, b = run("adamw", SHAPES, True), run("adamw", SHAPES, True, cuda_graph=True)
+    for x, y in zip(a, b):
+        assert float((x - y).norm()) <= 1e-6 * float(y.norm())
+
+
+def test_mixed_state_falls_back(native_lib):
+    """bf16 preconditioner state has no plan: the general path takes the step."""
+    from optimizers import shampoo2
+    p = torch.nn.Parameter(torch.randn(96, 80, device="cuda"))
+    opt = shampoo2.ShampooAdamW([p], prec_bits=16, stat_compute_steps=1, prec_compute_steps=1)
+    p.grad = torch.randn_like(p)
+    opt.step()
+    assert not opt._apply_plans and bool(torch.isfinite(p).all())
