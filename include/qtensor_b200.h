@@ -518,6 +518,29 @@ int qt_apply_group(void *out, const void *Ahi, const void *Alo, long long lda, l
                    void *D, long long ldd, int wide, float *part);
 int qt_apply_run(const qt_apply_desc *desc, void *stream);
 
+/*
+ * Refresh of one order class (64 <= n <= 1216, 4/8-bit eigen-factor statistics) as one host call: the statistics update
+ * (do_stat), then the inverse roots (do_root), for `count` consecutive matrices (optimizers/shampoo2.py:169-232).
+ *   gradients   groups of equally shaped blocks; their planes are made by work items (see qt_apply_run) that write at
+ *               byte offsets hi_off / lo_off of a region of grad_plane_bytes inside the workspace; `slots`: matrix of
+ *               each block; `first`: its index in gexp; axis 0: G G^T, 1: G^T G;
+ *   workspace   qt_refresh_workspace_bytes(desc) bytes of device memory (256-byte aligned), scratch.
+ * All strides of the state are contiguous per matrix: stride_codes bytes, n * ceil(n / blocksize) scales, n diagonal
+ * entries.  inv_p = 1/p of L^(-1/p).  Additive.
+ */
+typedef struct qt_refresh_group { const int *slots; long long hi_off, lo_off; int rows, cols, count, axis, first, reserved; } qt_refresh_group;
+typedef struct qt_refresh_desc {
+    const unsigned char *stat_codes; const float *stat_absmax; unsigned char *prec_codes; float *prec_absmax, *prec_diag;
+    float *S; long long *keep_idx; float *max_eig; const float *code;
+    const qt_refresh_group *groups; const void *grad_stat_items, *grad_split_items; const long long *grads;
+    float *part_amax, *part_ss; int *gexp;
+    long long stride_codes, grad_plane_bytes;
+    int n, count, keep, bits, blocksize, rect_t1, rect_t2, do_stat, do_root, n_groups, n_grad_stat, n_grad_split;
+    float w1, w2, eps, inv_p;
+} qt_refresh_desc;
+unsigned long long qt_refresh_workspace_bytes(const qt_refresh_desc *desc);
+int qt_refresh_class(const qt_refresh_desc *desc, void *workspace, unsigned long long workspace_bytes, void *stream);
+
 /* Sticky device-side error word (QT_OK or QT_ERR_TIMEOUT); synchronises the device.
  * clear != 0 resets it.  Additive; the reference has no device-side waits. */
 int qt_device_error(int clear);

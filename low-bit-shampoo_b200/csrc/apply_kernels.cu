@@ -187,7 +187,8 @@ __device__ __forceinline__ void store_f16_pair(__half *hi, __half *lo, const flo
 // two funnel shifts give the sixteen codes.
 __global__ void __launch_bounds__(kApplyThreads)
 k_apply_planes(const ApplyItem *__restrict__ items, const long long *__restrict__ grads, const float *__restrict__ code,
-               const float *__restrict__ part_amax, float *__restrict__ part_ss, const int *__restrict__ pexp, int *__restrict__ gexp, int target) {
+               const float *__restrict__ part_amax, float *__restrict__ part_ss, const int *__restrict__ pexp, int *__restrict__ gexp, int target,
+               long long plane_base) {
     __shared__ float red[kApplyThreads / 32];
     __shared__ __align__(16) unsigned char raw[2 * 32 * 33 * 4];
     float2 *pair_lut = reinterpret_cast<float2 *>(raw);
@@ -200,7 +201,7 @@ k_apply_planes(const ApplyItem *__restrict__ items, const long long *__restrict_
         if (it.p3 && threadIdx.x == 0) gexp[it.aux2] = e;     // the block's first item
         const float two_e = exp2f((float)e);
         const float *g = reinterpret_cast<const float *>(grads[it.param]) + it.off;
-        __half *hi = reinterpret_cast<__half *>(it.p0), *lo = reinterpret_cast<__half *>(it.p1);
+        __half *hi = reinterpret_cast<__half *>(plane_base + it.p0), *lo = reinterpret_cast<__half *>(plane_base + it.p1);
         const int rows = it.rows, cols = it.cols, ld = it.ld;
         const long long ldp = it.p2;
         const bool vec = (reinterpret_cast<uintptr_t>(g) & 31) == 0 && ld % 8 == 0;
@@ -604,6 +605,19 @@ k_apply_tail(const ApplyTailParams q) {
     }
 }
 
+// Gradient blocks as operand planes for the statistics: the pieces' magnitudes, then the planes at plane_base + the
+// items' offsets.
+int launch_grad_planes(const void *stat_items, int n_stat, const void *split_items, int n_split, const long long *grads, float *part_amax,
+                       float *part_ss, int *gexp, int target, void *plane_base, cudaStream_t s) {
+    if (n_stat <= 0 || n_split <= 0) return record(QT_OK);
+    if (!stat_items || !split_items || !grads || !part_amax || !part_ss || !gexp || !plane_base) return record(QT_ERR_ARG);
+    k_apply_stats<<<n_stat, kApplyThreads, 0, s>>>(static_cast<const ApplyItem *>(stat_items), grads, nullptr, part_amax, part_ss, nullptr, target);
+    k_apply_planes<<<n_split, kApplyThreads, 0, s>>>(static_cast<const ApplyItem *>(split_items), grads, nullptr, part_amax, part_ss, nullptr, gexp, target,
+                                                     reinterpret_cast<long long>(plane_base));
+    count_launch(2);
+    return check_launch();
+}
+
 static bool prepare_apply() {
     static PerDeviceOnce done;
     const int dev = current_device();
@@ -679,7 +693,7 @@ int qt_apply_run(const qt_apply_desc *d, void *stream) {
         if (v.n_groups > kMaxGroups) return record(QT_ERR_UNSUPPORTED);
         if (v.n_plane_items > 0) {
             k_apply_planes<<<v.n_plane_items, kApplyThreads, 0, s>>>(static_cast<const ApplyItem *>(v.plane_items), d->grads, d->code, d->part_amax,
-                                                                    d->part_ss, d->pexp, d->gexp, d->target);
+                                                                    d->part_ss, d->pexp, d->gexp, d->target, 0);
             count_launch(1);
         }
         if (v.n_groups > 0) {

@@ -24,6 +24,7 @@
 // Every wait is bounded: on expiry the kernel records an error word and drains.
 #include "quant_device.cuh"
 #include "tc_device.cuh"
+#include "gemm_api.cuh"
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cstring>
@@ -65,14 +66,6 @@ template <int NP, int BN_, int EC, bool CONV = false, bool PAIR = false> struct 
     static constexpr int NACC = TMEM_COLS / BN_;
 };
 
-// A product operand that lives as 4-bit blockwise state: matrix b of the product is state slot
-// slots[b] (null: b); its plane exponent is a_exp[b] / b_exp[b] of GemmParams.
-struct QOperand {
-    const unsigned char *codes; const float *absmax, *diag; const int *slots;
-    long long stride_codes, stride_absmax, stride_diag;                   // per slot: bytes, floats, floats
-    int n, nb;                                                            // order of the state matrices, blocks per row
-};
-
 struct GemmParams {
     int M, N, K, batch;
     float alpha, beta;
@@ -89,6 +82,9 @@ struct GemmParams {
     const int *out_exp; int *out_exp_w; int out_exp0, out_rel;            // exponent of the plane output: given per entry, or
                                                                           // (out_rel) operand exponents + out_exp0; written to out_exp_w
     int kc;                                                               // k-blocks per accumulation chain (two-plane kernels)
+    int sym;                                                              // only tiles on and above the diagonal are computed; the others are mirrored
+    float *amax_out;                                                      // per output entry: max |result| (atomic max)
+    float *cd_part;                                                       // column sums of result * C per 32 rows, instead of a stored result
     int c_follows_d;                                                      // C of matrix b is entry d_slot[b] of its array (in-place updates of selected entries)
     // Operands taken straight from 4-bit state (CONV kernels; block size 64, square order qn):
     // codes == nullptr: the operand comes from its planes through TMA as usual.
@@ -101,6 +97,17 @@ struct GemmParams {
     long long q_stride_codes, q_stride_absmax, q_stride_diag;             // per matrix: bytes, floats, floats
     const float *q_code; int q_nb;
 };
+
+// Symmetric result: tile number -> (row band, column band) with row band <= column band.
+__device__ __forceinline__ void tile_coords_sym(int tile, int tiles, int &tm, int &tn, int &b) {
+    const int per_matrix = tiles * (tiles + 1) / 2;
+    b = tile / per_matrix;
+    const int t = tile - b * per_matrix;
+    tn = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    if ((tn + 1) * (tn + 2) / 2 <= t) ++tn;
+    if (tn * (tn + 1) / 2 > t) --tn;
+    tm = t - tn * (tn + 1) / 2;
+}
 
 template <bool Q> struct QuantTablesHolder { CodeTables<16> t; };
 template <> struct QuantTablesHolder<false> { int unused; };
@@ -281,6 +288,35 @@ __device__ __forceinline__ void store_planes_f16(__half *hi, __half *lo, const f
     }
 }
 
+// The same 16 values as one column each of the mirrored tile (row pitch ld): 64 contiguous bytes per warp, column and plane.
+template <int NP>
+__device__ __forceinline__ void store_planes_mirrored(__nv_bfloat16 *hi, __nv_bfloat16 *mid, __nv_bfloat16 *lo, const float (&v)[16], long long ld,
+                                                      float scale, bool f16, int nvalid) {
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        if (t < nvalid) {
+            if (NP == 2 && f16) {
+                float x = fminf(fmaxf(v[t] * scale, -65000.0f), 65000.0f);    // the direct store reports a clamped value
+                if (!(x == x)) x = 0.0f;
+                const __half h = __float2half_rn(x);
+                reinterpret_cast<__half *>(hi)[t * ld] = h;
+                reinterpret_cast<__half *>(lo)[t * ld] = __float2half_rn(x - __half2float(h));
+            } else {
+                const __nv_bfloat16 h = __float2bfloat16_rn(v[t]);
+                const float r1 = v[t] - __bfloat162float(h);
+                const __nv_bfloat16 m = __float2bfloat16_rn(r1);
+                hi[t * ld] = h;
+                if constexpr (NP == 3) {
+                    mid[t * ld] = m;
+                    lo[t * ld] = __float2bfloat16_rn(r1 - __bfloat162float(m));
+                } else {
+                    lo[t * ld] = m;
+                }
+            }
+        }
+    }
+}
+
 // 64 consecutive elements of row `row` of a 4-bit state matrix, starting at column `col` (a
 // multiple of 64: exactly one quantization block), dequantized exactly as k_dequantize_planes
 // does (code * scale, fp32 diagonal restored), scaled by two_e and split into fp16 hi / lo;
@@ -380,7 +416,7 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
     // (not in a pair: the two CTAs could decide differently, and one would wait for the other)
     if (!PAIR && *reinterpret_cast<volatile int *>(&g_gemm_error) != 0) return;
     const int num_kb = (p.K + BK - 1) / BK;
-    const int num_tiles = p.tiles_m * p.tiles_n * p.batch;
+    const int num_tiles = (p.sym ? p.tiles_m * (p.tiles_m + 1) / 2 : p.tiles_m * p.tiles_n) * p.batch;
     const int nchunks = (num_kb + KC - 1) / KC;
 
     const bool conv_a = CONV && p.aq.codes != nullptr, conv_b = CONV && p.bq.codes != nullptr;
@@ -414,6 +450,10 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
         __syncthreads();
     }
 
+    auto coords = [&](int tile, int &tm, int &tn, int &b) {
+        if (!PAIR && p.sym) tile_coords_sym(tile, p.tiles_m, tm, tn, b);
+        else tile_coords<PAIR ? RASTER_M / 2 : RASTER_M>(tile, p.tiles_m, p.tiles_n, tm, tn, b);
+    };
     // A matrix whose entry of `active` is zero is skipped by all three roles alike (the array
     // does not change while the kernel runs), so their ring and accumulator counters stay in step.
     auto skipped = [&](int b) { return p.active != nullptr && __ldg(p.active + b) == 0; };
@@ -425,7 +465,7 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
             bool ok = true;
             for (int tile = cta_first; tile < num_tiles && ok; tile += cta_step) {
                 int tm, tn, b;
-                tile_coords<PAIR ? RASTER_M / 2 : RASTER_M>(tile, p.tiles_m, p.tiles_n, tm, tn, b);
+                coords(tile, tm, tn, b);
                 if (skipped(b)) continue;
                 const int za = p.a_slot ? __ldg(p.a_slot + b) : b;
                 const int zb = p.b_slot ? __ldg(p.b_slot + b) : b;
@@ -505,7 +545,7 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
                 // a ragged last column band needs only its own columns (N is any multiple of 16):
                 // the tensor core's time per MMA scales with N
                 int tm_, tn_, b_;
-                tile_coords<PAIR ? RASTER_M / 2 : RASTER_M>(tile, p.tiles_m, p.tiles_n, tm_, tn_, b_);
+                coords(tile, tm_, tn_, b_);
                 if (skipped(b_)) continue;
                 const int ncur = min(BN_, (p.N - tn_ * BN_ + 15) & ~15);
                 const unsigned idesc_tile = (idesc & ~(0x3Fu << 17)) | ((unsigned)(ncur >> 3) << 17);
@@ -576,7 +616,7 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
         const unsigned lead_acc_empty0 = PAIR ? map_to_cta(acc_empty(0), 0u) : 0u;
         for (int tile = cta_first; tile < num_tiles; tile += cta_step) {
             int tm, tn, b;
-            tile_coords<PAIR ? RASTER_M / 2 : RASTER_M>(tile, p.tiles_m, p.tiles_n, tm, tn, b);
+            coords(tile, tm, tn, b);
             if (skipped(b)) continue;
             if constexpr (PAIR) tm = 2 * tm + (int)rank;       // this CTA's 128-row band
             const int m0 = tm * BM, n0 = tn * BN_ + seg * EC;
@@ -628,6 +668,43 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
                     pscale = exp2f((float)e_out);
                     if (p.out_exp_w && tm == 0 && tn == 0 && seg == 0 && quad == 0 && lane == 0) p.out_exp_w[bo] = e_out;
                 }
+                if (NP == 2 && EC <= 96 && p.cd_part) {
+                    // sum over the warp's 32 rows of result * C for every column: sixteen columns at a time are reduced and
+                    // scattered over the lanes (16 shuffles), in an order that depends on the shape only
+                    const float *crow = p.C + (long long)b * p.strideC + (long long)row * p.ldc + n0;
+                    float *part = p.cd_part + ((long long)b * (4 * p.tiles_m) + tm * 4 + quad) * p.N + n0;
+#pragma unroll
+                    for (int q = 0; q < EC; q += 16) {
+                        if (q >= valid) continue;
+                        float o[16];
+#pragma unroll
+                        for (int t = 0; t < 16; ++t) o[t] = 0.0f;
+                        if (row_ok) {
+                            if (q + 16 <= valid && wide_d) { ldg256f(crow + q, o); ldg256f(crow + q + 8, o + 8); }
+                            else {
+#pragma unroll
+                                for (int t = 0; t < 16; ++t) if (q + t < valid) o[t] = __ldg(crow + q + t);
+                            }
+                        }
+#pragma unroll
+                        for (int t = 0; t < 16; ++t) o[t] *= alpha_eff * sum[q + t];
+#pragma unroll
+                        for (int w = 8; w >= 1; w >>= 1) {
+                            const bool upper = (lane & (2 * w)) != 0;
+#pragma unroll
+                            for (int t = 0; t < w; ++t) {
+                                const float keep = upper ? o[t + w] : o[t], give = upper ? o[t] : o[t + w];
+                                o[t] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * w);
+                            }
+                        }
+                        o[0] += __shfl_xor_sync(0xffffffffu, o[0], 1);
+                        const int col = q + (lane >> 1);       // lane bits 4..1 chose the column
+                        if ((lane & 1) == 0 && col < valid) part[col] = o[0];
+                    }
+                    continue;
+                }
+                const bool mirror = p.sym && tm != tn;
+                float amax = 0.0f;                              // max |result| over this thread's elements
                 if (row_ok && valid > 0) {
                     const float *crow = p.C + (long long)(p.c_follows_d ? bo : b) * p.strideC + (long long)row * p.ldc + n0;
                     float *drow = p.D + (long long)bo * p.strideD + (long long)row * p.ldd + n0;
@@ -670,6 +747,19 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
 #pragma unroll
                                 for (int t = 0; t < 16; ++t) if (q + t < valid) drow[q + t] = o[t];
                             }
+                            if (mirror) {                       // lanes hold consecutive rows: 128 contiguous bytes per column
+                                float *dcol = p.D + (long long)bo * p.strideD + (long long)(n0 + q) * p.ldd + row;
+#pragma unroll
+                                for (int t = 0; t < 16; ++t) if (q + t < valid) dcol[(long long)t * p.ldd] = o[t];
+                            }
+                        }
+                        if (p.amax_out) {
+#pragma unroll
+                            for (int t = 0; t < 16; ++t) if (q + t < valid) amax = fmaxf(amax, fabsf(o[t]));
+                        }
+                        if (p.Dhi && mirror) {
+                            const long long pm = (long long)bo * p.strideP + (long long)(n0 + q) * p.ldp + row;
+                            store_planes_mirrored<NP>(p.Dhi + pm, NP == 3 ? p.Dmid + pm : nullptr, p.Dlo + pm, o, p.ldp, pscale, NP == 2 && p.f16, valid - q);
                         }
                         if (p.Dhi) {
                             if (NP == 2 && p.f16)
@@ -696,9 +786,18 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
 #pragma unroll
                                 for (int t = 0; t < 16; ++t) tv[t] = fmaf(p.t_c1, o[t], t == dcol ? p.t_c0 : 0.0f);
                                 store_planes<3>(p.Thi + to + q, p.Tmid + to + q, p.Tlo + to + q, tv, full16 && wide_p, valid - q);
+                                if (mirror) {
+                                    const long long tmr = (long long)b * p.strideP + (long long)(n0 + q) * p.ldp + row;
+                                    store_planes_mirrored<3>(p.Thi + tmr, p.Tmid + tmr, p.Tlo + tmr, tv, p.ldp, 1.0f, false, valid - q);
+                                }
                             }
                         }
                     }
+                }
+                if (p.amax_out) {
+#pragma unroll
+                    for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+                    if (lane == 0 && amax > 0.0f) atomicMax(reinterpret_cast<int *>(p.amax_out + bo), __float_as_int(amax));
                 }
                 if (p.maxdev) {
 #pragma unroll
@@ -1131,45 +1230,7 @@ int launch_split_bf16_3(const float *X, long long ldx, long long strideX, int ro
     return check_launch();
 }
 
-struct GemmArgs {
-    const void *Ahi, *Alo; long long lda, strideA; int a_mn;
-    const void *Bhi, *Blo; long long ldb, strideB; int b_mn;
-    int M, N, K, batch; float alpha, beta;
-    const float *C; long long ldc, strideC;
-    float *D; long long ldd, strideD;
-    void *Dhi, *Dlo; long long ldp, strideP;
-};
-
-// Optional extras of a product (all pointers device memory, any of them may be null).
-struct GemmExtras {
-    void *Dmid = nullptr;                                   // middle result plane (three-plane products)
-    void *Thi = nullptr, *Tmid = nullptr, *Tlo = nullptr;   // t_c0 * I + t_c1 * result, three planes (pitch of the result planes)
-    float t_c0 = 0.0f, t_c1 = 0.0f;
-    float *maxdev = nullptr;                                // per matrix max |result - I|
-    const int *a_slot = nullptr, *b_slot = nullptr, *d_slot = nullptr;
-    const int *active = nullptr;
-    int a_entries = 0, b_entries = 0;                       // matrices in A's / B's storage (0: batch)
-    // scaled fp16 planes (two-plane products only)
-    int f16 = 0;
-    const int *a_exp = nullptr, *b_exp = nullptr; int ab_exp0 = 0;
-    const int *out_exp = nullptr; int *out_exp_w = nullptr; int out_exp0 = 0, out_rel = 0;
-    int kc = 0;                                             // k-blocks per accumulation chain (0: one chain)
-    // operands straight from 4-bit state (see QOperand); codes == nullptr: from planes
-    QOperand aq = {nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0}, bq = {nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0};
-    const float *oq_code = nullptr;
-    int max_ctas = 0;                                       // > 0: cap of the persistent grid (SMs left to kernels on other streams)
-    int c_follows_d = 0;                                    // C indexed through d_slot like the outputs
-};
-
 static inline bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
-// 4-bit state operands of the quantizing variant (all device pointers; see GemmParams).
-struct QuantStateArgs {
-    const float *code;
-    const unsigned char *q_in; const float *absmax_in, *diag_in;
-    unsigned char *q_out; float *absmax_out, *diag_out;
-    long long stride_codes, stride_absmax, stride_diag;
-};
 
 typedef void (*GemmKern)(const GemmMaps, const GemmParams);
 
@@ -1229,10 +1290,8 @@ static bool prepare_kernels() {
 // with that tile width; 512: CTA pairs wherever they are possible.
 static int g_force_bn = -1;
 
-// a.Ahi/Alo (+ Amid/Bmid for three planes: order hi, mid, lo).  With `qs` the result (and the C
-// operand, if qs->q_in) is 4-bit state instead of a.C / a.D.
 int launch_gemm_planes(const GemmArgs &a, const void *Amid, const void *Bmid, cudaStream_t s, const QuantStateArgs *qs,
-                       const GemmExtras *ex = nullptr) {
+                       const GemmExtras *ex) {
     const int np = (Amid && Bmid) ? 3 : 2;
     static const GemmExtras none;
     const GemmExtras &x = ex ? *ex : none;
@@ -1256,13 +1315,15 @@ int launch_gemm_planes(const GemmArgs &a, const void *Amid, const void *Bmid, cu
         if ((qa && ((reinterpret_cast<uintptr_t>(x.aq.codes) & 7) || (x.aq.stride_codes & 7))) ||
             (qb && ((reinterpret_cast<uintptr_t>(x.bq.codes) & 7) || (x.bq.stride_codes & 7)))) return record(QT_ERR_ARG);
     }
-    if ((!qa && (!a.Ahi || !a.Alo)) || (!qb && (!a.Bhi || !a.Blo)) || (!qs && !a.D && !a.Dhi && !x.Thi && !x.maxdev)) return record(QT_ERR_ARG);
+    if ((!qa && (!a.Ahi || !a.Alo)) || (!qb && (!a.Bhi || !a.Blo)) || (!qs && !a.D && !a.Dhi && !x.Thi && !x.maxdev && !x.cd_part)) return record(QT_ERR_ARG);
     if ((a.Dhi == nullptr) != (a.Dlo == nullptr) || (Amid == nullptr) != (Bmid == nullptr)) return record(QT_ERR_ARG);
     if (a.Dhi && np == 3 && !x.Dmid) return record(QT_ERR_ARG);                  // three-plane result needs all three planes
     if (x.Thi && (!x.Tmid || !x.Tlo || np != 3 || a.ldp <= 0)) return record(QT_ERR_ARG);
     if ((x.Thi || x.maxdev || x.Dmid) && qs) return record(QT_ERR_UNSUPPORTED);
     if (x.f16 && np != 2) return record(QT_ERR_UNSUPPORTED);
     if (x.kc < 0) return record(QT_ERR_ARG);
+    if (x.sym && (a.M != a.N || qs || x.aq.codes || x.bq.codes)) return record(QT_ERR_UNSUPPORTED);
+    if (x.cd_part && (np != 2 || qs || !a.C || a.D || a.Dhi || x.sym || x.aq.codes || x.bq.codes)) return record(QT_ERR_UNSUPPORTED);
     const int a_entries = x.a_entries > 0 ? x.a_entries : a.batch, b_entries = x.b_entries > 0 ? x.b_entries : a.batch;
     const void *Ap[3] = {a.Ahi, np == 3 ? Amid : a.Alo, a.Alo};
     const void *Bp[3] = {a.Bhi, np == 3 ? Bmid : a.Blo, a.Blo};
@@ -1281,7 +1342,7 @@ int launch_gemm_planes(const GemmArgs &a, const void *Amid, const void *Bmid, cu
     // registers a 320-thread CTA leaves them; over the whole optimizer step it loses 0.6 ms.  It
     // stays selectable (qt_gemm_force_tile) for measurements.
     int cfg = np == 3 ? 2 : 0;
-    if (np == 2 && a.N > 128 && g_force_bn == 256) cfg = 1;
+    if (np == 2 && a.N > 128 && g_force_bn == 256 && !x.sym && !x.cd_part) cfg = 1;
     // 128 x 192 tiles (eight epilogue warps of 96 columns, two operand stages, two accumulators): 17 % less
     // operand traffic per flop than 128 x 128 and, unlike 128 x 256, the 96 partial sums per thread
     // (nearly) fit the register budget.  Measured against 128 x 128: 125 x 768^3 371 -> 332 us,
@@ -1290,20 +1351,20 @@ int launch_gemm_planes(const GemmArgs &a, const void *Amid, const void *Bmid, cu
     // Products whose epilogue reads C and writes both fp32 and planes stay on 128 x 128 as well (the wide
     // epilogue is out of registers there: 600 x 1200 x 600 with all three 1.01 -> 1.10 ms per four launches).
     const bool heavy_epilogue = a.C && a.beta != 0.0f && a.D && a.Dhi;
-    if (np == 2 && a.N > 128 && !qs && (g_force_bn == 192 || (g_force_bn == -1 && a.K >= 256 && !heavy_epilogue))) cfg = 5;
+    if (np == 2 && a.N > 128 && !qs && !x.sym && (g_force_bn == 192 || (g_force_bn == -1 && a.K >= 256 && !heavy_epilogue))) cfg = 5;
     if (qa || qb) cfg = 3;
     // CTA pairs (256-row bands) only on request: measured on B200 they are no faster than single
     // CTAs on 128 x 128 tiles (125 x 768^3: 372 vs 364 us; 8 x 4096^3: 3980 vs 3480 us) - halving
     // the B operand a CTA stages does not pay while each SM still multiplies 128 x 128 x 16 per
     // instruction; the 128 x 256 single-CTA tile is the one that gains (2900 us on the large case).
-    const bool pair_possible = cfg == 0 && !qs && sms >= 2 && a.M > BM;
+    const bool pair_possible = cfg == 0 && !qs && !x.sym && !x.cd_part && sms >= 2 && a.M > BM;
     if (pair_possible && g_force_bn == 512) cfg = 4;
     const bool pair = cfg == 4;
     const int bn = g_cfg_bn[cfg];
     GemmMaps maps;
     memset(&maps, 0, sizeof(maps));
     bool ok = true;
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < np; ++i) {
         const void *pa = Ap[i < np ? i : 0], *pb = Bp[i < np ? i : 0];
         const bool h = x.f16 != 0;
         if (qa) {}
@@ -1326,6 +1387,7 @@ int launch_gemm_planes(const GemmArgs &a, const void *Amid, const void *Bmid, cu
     p.f16 = x.f16; p.a_exp = x.a_exp; p.b_exp = x.b_exp; p.ab_exp0 = x.ab_exp0;
     p.out_exp = x.out_exp; p.out_exp_w = x.out_exp_w; p.out_exp0 = x.out_exp0; p.out_rel = x.out_rel; p.kc = x.kc; p.c_follows_d = x.c_follows_d;
     p.aq = x.aq; p.bq = x.bq; p.oq_code = x.oq_code;
+    p.sym = x.sym; p.amax_out = x.amax_out; p.cd_part = x.cd_part;
     p.tiles_m = pair ? (a.M + 2 * BM - 1) / (2 * BM) : tiles_m; p.tiles_n = (a.N + bn - 1) / bn;
     p.q_in = nullptr; p.q_absmax_in = p.q_diag_in = nullptr; p.q_out = nullptr; p.q_absmax_out = p.q_diag_out = nullptr;
     p.q_stride_codes = p.q_stride_absmax = p.q_stride_diag = 0; p.q_code = nullptr; p.q_nb = 0;
@@ -1335,7 +1397,7 @@ int launch_gemm_planes(const GemmArgs &a, const void *Amid, const void *Bmid, cu
         p.q_stride_codes = qs->stride_codes; p.q_stride_absmax = qs->stride_absmax; p.q_stride_diag = qs->stride_diag;
         p.q_code = qs->code; p.q_nb = (a.N + 63) / 64;
     }
-    const long long ctas = (long long)p.tiles_m * p.tiles_n * a.batch;
+    const long long ctas = (x.sym ? (long long)p.tiles_m * (p.tiles_m + 1) / 2 : (long long)p.tiles_m * p.tiles_n) * a.batch;
     if (ctas > 0x7fffffffLL) return record(QT_ERR_UNSUPPORTED);
     GemmKern kern = g_kernels[cfg][a.a_mn ? 1 : 0][a.b_mn ? 1 : 0][qs ? 1 : 0];
     if (pair) {
@@ -1602,8 +1664,8 @@ int qt_matmul_f32_static(const float *A, long long lda, long long strideA, int t
 }
 
 int qt_device_error(int clear) {
-    const int a = read_gemm_error(clear != 0), b = read_apply_error(clear != 0);
-    return a != 0 ? a : b;
+    const int e[3] = {read_gemm_error(clear != 0), read_apply_error(clear != 0), read_refresh_error(clear != 0)};
+    return e[0] != 0 ? e[0] : e[1] != 0 ? e[1] : e[2];
 }
 
 void qt_gemm_force_tile(int bn) { g_force_bn = bn; }

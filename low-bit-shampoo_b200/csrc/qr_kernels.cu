@@ -11,9 +11,27 @@
 // Conventions are LAPACK's (slarfg / slarft, forward, columnwise): beta = -sign(alpha)
 // * ||x||, tau = (beta - alpha) / beta, v = x / (alpha - beta) with v_0 = 1; a column
 // that is already zero below the diagonal gets tau = 0.
-#include "qt_common.cuh"
+#include "quant_device.cuh"
+#include <cuda_fp16.h>
 
 namespace qt {
+
+// Operand planes of an outer block's Householder vectors, written by the panel kernels beside V itself: scaled fp16
+// pairs (entries <= 1, so the exponent is fixed), [matrix][n - J0 rows][pitch ld], the panel's columns at col0.  Rows above
+// the panel inside the block are written as zeros.
+struct PanelPlanes { __half *hi, *lo; long long ld, stride; int col0, rows_above; float scale; };
+
+__device__ __forceinline__ void store_panel_planes(const PanelPlanes &pp, const float *P, int m, int w, int warps) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!pp.hi || lane >= w) return;
+    __half *hi = pp.hi + (long long)blockIdx.x * pp.stride + pp.col0 + lane, *lo = pp.lo + (long long)blockIdx.x * pp.stride + pp.col0 + lane;
+    for (int r = warp; r < m + pp.rows_above; r += warps) {
+        const float x = r < pp.rows_above ? 0.0f : P[(r - pp.rows_above) * 33 + lane] * pp.scale;
+        const __half h = __float2half_rn(x);
+        hi[(long long)r * pp.ld] = h;
+        lo[(long long)r * pp.ld] = __float2half_rn(x - __half2float(h));
+    }
+}
 
 static constexpr int kPanel = 32;
 static constexpr int kQrThreads = 1024;                    // one warp per panel column
@@ -46,9 +64,9 @@ __device__ __forceinline__ float warp_sum(float v) {
 // panel that a separate rank-32 update needs, and the CTAs of chunks 1.. fill otherwise idle SMs.
 template <int RPL, int RS>
 __global__ void __launch_bounds__(kQrThreads, 1)
-k_householder_panel(float *__restrict__ Abase, long long strideA, int n, int j0, int w,
+k_householder_panel(float *__restrict__ Abase, long long strideA, int n, int ld, int j0, int w,
                     float *__restrict__ Vbase, long long strideV, float *__restrict__ Tbase, long long strideT,
-                    int prev_w, const float *__restrict__ Tprev_base, int block_end) {
+                    int prev_w, const float *__restrict__ Tprev_base, int block_end, const PanelPlanes planes) {
     constexpr int RT = RPL + RS;
     extern __shared__ float sm[];
     const int m = n - j0;
@@ -64,7 +82,7 @@ k_householder_panel(float *__restrict__ Abase, long long strideA, int n, int j0,
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int chunk = blockIdx.y;
     float *Amat = Abase + (long long)blockIdx.x * strideA;
-    const float *A = Amat + (long long)j0 * n + j0;
+    const float *A = Amat + (long long)j0 * ld + j0;
 
     if (prev_w > 0) {
         // ---- apply the previous panel's block reflector to this CTA's column chunk
@@ -73,9 +91,9 @@ k_householder_panel(float *__restrict__ Abase, long long strideA, int n, int j0,
         const int c0 = j0 + kPanel * chunk;                // first column of the chunk
         const int wc = min(kPanel, block_end - c0);        // columns of the chunk
         float *C = Pall + (kPanel - prev_w) * 33;          // window rows so that row prev_w of it is P's row 0
-        float *Cg = Amat + (long long)r0 * n + c0;
-        const float *Vg = Vbase + (long long)blockIdx.x * strideV + (long long)r0 * n + r0;
-        for (int r = warp; r < mu; r += 32) C[r * 33 + lane] = (lane < wc) ? Cg[(long long)r * n + lane] : 0.0f;
+        float *Cg = Amat + (long long)r0 * ld + c0;
+        const float *Vg = Vbase + (long long)blockIdx.x * strideV + (long long)r0 * ld + r0;
+        for (int r = warp; r < mu; r += 32) C[r * 33 + lane] = (lane < wc) ? Cg[(long long)r * ld + lane] : 0.0f;
         for (int i = tid; i < kPanel * kPanel; i += kQrThreads) {
             const int a = i / kPanel, b = i - a * kPanel;
             Tp[a * (kPanel + 1) + b] = (a < prev_w && b < prev_w) ? Tprev_base[(long long)blockIdx.x * strideT + i] : 0.0f;
@@ -92,7 +110,7 @@ k_householder_panel(float *__restrict__ Abase, long long strideA, int n, int j0,
 #pragma unroll
             for (int q = 0; q < kPer; ++q) {
                 const int i = tid + q * kQrThreads, rr = i >> 5, j = i & 31;
-                pre[q] = (rb + rr < mu && j < prev_w) ? Vg[(long long)(rb + rr) * n + j] : 0.0f;
+                pre[q] = (rb + rr < mu && j < prev_w) ? Vg[(long long)(rb + rr) * ld + j] : 0.0f;
             }
         };
         auto stash = [&]() {
@@ -177,14 +195,14 @@ k_householder_panel(float *__restrict__ Abase, long long strideA, int n, int j0,
         __syncthreads();
         if (chunk > 0) {                                   // not the new panel: write the updated chunk back and leave
             for (int r = warp; r < mu; r += 32)
-                if (lane < wc) Cg[(long long)r * n + lane] = C[r * 33 + lane];
+                if (lane < wc) Cg[(long long)r * ld + lane] = C[r * 33 + lane];
             return;
         }
         // chunk 0: rows prev_w.. of the window are the new panel, already in P
         for (int r = warp; r < m; r += 32)
             if (lane >= w) P[r * 33 + lane] = 0.0f;
     } else {
-        for (int r = warp; r < m; r += 32) P[r * 33 + lane] = (lane < w) ? A[(long long)r * n + lane] : 0.0f;
+        for (int r = warp; r < m; r += 32) P[r * 33 + lane] = (lane < w) ? A[(long long)r * ld + lane] : 0.0f;
     }
     for (int i = tid; i < 2 * kPanel * (kPanel + 1); i += kQrThreads) G[i] = 0.0f;   // G and Ts are adjacent
     __syncthreads();
@@ -294,9 +312,10 @@ k_householder_panel(float *__restrict__ Abase, long long strideA, int n, int j0,
         if (r < m) P[r * 33 + warp] = col[k];
     }
     __syncthreads();
-    float *V = Vbase + (long long)blockIdx.x * strideV + (long long)j0 * n + j0;
+    float *V = Vbase + (long long)blockIdx.x * strideV + (long long)j0 * ld + j0;
     for (int r = warp; r < m; r += 32)
-        if (lane < w) V[(long long)r * n + lane] = P[r * 33 + lane];
+        if (lane < w) V[(long long)r * ld + lane] = P[r * 33 + lane];
+    store_panel_planes(planes, P, m, w, 32);
     float *T = Tbase + (long long)blockIdx.x * strideT;
     for (int i = tid; i < kPanel * kPanel; i += kQrThreads) T[i] = Ts[(i / kPanel) * (kPanel + 1) + (i % kPanel)];
 }
@@ -311,9 +330,9 @@ k_householder_panel(float *__restrict__ Abase, long long strideA, int n, int j0,
 // previous panel, same outputs as k_householder_panel.
 template <int RT>
 __global__ void __launch_bounds__(512, 1)
-k_householder_panel_pairs(float *__restrict__ Abase, long long strideA, int n, int j0, int w,
+k_householder_panel_pairs(float *__restrict__ Abase, long long strideA, int n, int ld, int j0, int w,
                           float *__restrict__ Vbase, long long strideV, float *__restrict__ Tbase, long long strideT,
-                          int prev_w, const float *__restrict__ Tprev_base, int block_end) {
+                          int prev_w, const float *__restrict__ Tprev_base, int block_end, const PanelPlanes planes) {
     constexpr int NW = 16, NT = NW * 32;
     extern __shared__ float sm[];
     const int m = n - j0;
@@ -329,7 +348,7 @@ k_householder_panel_pairs(float *__restrict__ Abase, long long strideA, int n, i
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int chunk = blockIdx.y;
     float *Amat = Abase + (long long)blockIdx.x * strideA;
-    const float *A = Amat + (long long)j0 * n + j0;
+    const float *A = Amat + (long long)j0 * ld + j0;
 
     if (prev_w > 0) {
         // ---- apply the previous panel's block reflector to this CTA's column chunk
@@ -338,9 +357,9 @@ k_householder_panel_pairs(float *__restrict__ Abase, long long strideA, int n, i
         const int c0 = j0 + kPanel * chunk;                // first column of the chunk
         const int wc = min(kPanel, block_end - c0);        // columns of the chunk
         float *C = Pall + (kPanel - prev_w) * 33;          // window rows so that row prev_w of it is P's row 0
-        float *Cg = Amat + (long long)r0 * n + c0;
-        const float *Vg = Vbase + (long long)blockIdx.x * strideV + (long long)r0 * n + r0;
-        for (int r = warp; r < mu; r += NW) C[r * 33 + lane] = (lane < wc) ? Cg[(long long)r * n + lane] : 0.0f;
+        float *Cg = Amat + (long long)r0 * ld + c0;
+        const float *Vg = Vbase + (long long)blockIdx.x * strideV + (long long)r0 * ld + r0;
+        for (int r = warp; r < mu; r += NW) C[r * 33 + lane] = (lane < wc) ? Cg[(long long)r * ld + lane] : 0.0f;
         for (int i = tid; i < kPanel * kPanel; i += NT) {
             const int a = i / kPanel, b = i - a * kPanel;
             Tp[a * (kPanel + 1) + b] = (a < prev_w && b < prev_w) ? Tprev_base[(long long)blockIdx.x * strideT + i] : 0.0f;
@@ -357,7 +376,7 @@ k_householder_panel_pairs(float *__restrict__ Abase, long long strideA, int n, i
 #pragma unroll
             for (int q = 0; q < kPer; ++q) {
                 const int i = tid + q * NT, rr = i >> 5, j = i & 31;
-                pre[q] = (rb + rr < mu && j < prev_w) ? Vg[(long long)(rb + rr) * n + j] : 0.0f;
+                pre[q] = (rb + rr < mu && j < prev_w) ? Vg[(long long)(rb + rr) * ld + j] : 0.0f;
             }
         };
         auto stash = [&]() {
@@ -443,14 +462,14 @@ k_householder_panel_pairs(float *__restrict__ Abase, long long strideA, int n, i
         __syncthreads();
         if (chunk > 0) {                                   // not the new panel: write the updated chunk back and leave
             for (int r = warp; r < mu; r += NW)
-                if (lane < wc) Cg[(long long)r * n + lane] = C[r * 33 + lane];
+                if (lane < wc) Cg[(long long)r * ld + lane] = C[r * 33 + lane];
             return;
         }
         // chunk 0: rows prev_w.. of the window are the new panel, already in P
         for (int r = warp; r < m; r += NW)
             if (lane >= w) P[r * 33 + lane] = 0.0f;
     } else {
-        for (int r = warp; r < m; r += NW) P[r * 33 + lane] = (lane < w) ? A[(long long)r * n + lane] : 0.0f;
+        for (int r = warp; r < m; r += NW) P[r * 33 + lane] = (lane < w) ? A[(long long)r * ld + lane] : 0.0f;
     }
     for (int i = tid; i < 2 * kPanel * (kPanel + 1); i += NT) G[i] = 0.0f;   // G and Ts are adjacent
     __syncthreads();
@@ -544,17 +563,18 @@ k_householder_panel_pairs(float *__restrict__ Abase, long long strideA, int n, i
         if (r < m) { P[r * 33 + cA] = colA[k]; P[r * 33 + cB] = colB[k]; }
     }
     __syncthreads();
-    float *V = Vbase + (long long)blockIdx.x * strideV + (long long)j0 * n + j0;
+    float *V = Vbase + (long long)blockIdx.x * strideV + (long long)j0 * ld + j0;
     for (int r = warp; r < m; r += NW)
-        if (lane < w) V[(long long)r * n + lane] = P[r * 33 + lane];
+        if (lane < w) V[(long long)r * ld + lane] = P[r * 33 + lane];
+    store_panel_planes(planes, P, m, w, NW);
     float *T = Tbase + (long long)blockIdx.x * strideT;
     for (int i = tid; i < kPanel * kPanel; i += NT) T[i] = Ts[(i / kPanel) * (kPanel + 1) + (i % kPanel)];
 }
 
 template <int RPL, int RS>
-static int launch_panel_rpl(float *A, long long strideA, int n, int count, int j0, int w,
+static int launch_panel_rpl(float *A, long long strideA, int n, int ld, int count, int j0, int w,
                             float *V, long long strideV, float *T, long long strideT, cudaStream_t s,
-                            int prev_w, const float *Tprev, int block_end) {
+                            int prev_w, const float *Tprev, int block_end, const PanelPlanes &planes) {
     const int m = n - j0;
     const size_t smem = sizeof(float) * ((size_t)(((kPanel + m) * 33 + 31) & ~31) + 2 * (RPL + RS) * 32 + 2 * kPanel * (kPanel + 1) + kPanel +
                                          256 * 36 + kPanel * (kPanel + 1) + kPanel * (kPanel + 1));
@@ -568,15 +588,15 @@ static int launch_panel_rpl(float *A, long long strideA, int n, int count, int j
     if (smem > 227 * 1024) return record(QT_ERR_UNSUPPORTED);
     const int chunks = prev_w > 0 ? (block_end - j0 + kPanel - 1) / kPanel : 1;
     dim3 grid(count, chunks);
-    k_householder_panel<RPL, RS><<<grid, kQrThreads, smem, s>>>(A, strideA, n, j0, w, V, strideV, T, strideT, prev_w, Tprev, block_end);
+    k_householder_panel<RPL, RS><<<grid, kQrThreads, smem, s>>>(A, strideA, n, ld, j0, w, V, strideV, T, strideT, prev_w, Tprev, block_end, planes);
     count_launch(1);
     return check_launch();
 }
 
 template <int RT>
-static int launch_panel_pairs(float *A, long long strideA, int n, int count, int j0, int w,
+static int launch_panel_pairs(float *A, long long strideA, int n, int ld, int count, int j0, int w,
                               float *V, long long strideV, float *T, long long strideT, cudaStream_t s,
-                              int prev_w, const float *Tprev, int block_end) {
+                              int prev_w, const float *Tprev, int block_end, const PanelPlanes &planes) {
     const int m = n - j0;
     const size_t smem = sizeof(float) * ((size_t)(((kPanel + m) * 33 + 31) & ~31) + 2 * RT * 32 + 2 * kPanel * (kPanel + 1) + kPanel +
                                          256 * 36 + kPanel * (kPanel + 1) + kPanel * (kPanel + 1));
@@ -590,15 +610,18 @@ static int launch_panel_pairs(float *A, long long strideA, int n, int count, int
     if (smem > 227 * 1024) return record(QT_ERR_UNSUPPORTED);
     const int chunks = prev_w > 0 ? (block_end - j0 + kPanel - 1) / kPanel : 1;
     dim3 grid(count, chunks);
-    k_householder_panel_pairs<RT><<<grid, 512, smem, s>>>(A, strideA, n, j0, w, V, strideV, T, strideT, prev_w, Tprev, block_end);
+    k_householder_panel_pairs<RT><<<grid, 512, smem, s>>>(A, strideA, n, ld, j0, w, V, strideV, T, strideT, prev_w, Tprev, block_end, planes);
     count_launch(1);
     return check_launch();
 }
 
-int launch_householder_panel(float *A, long long strideA, int n, int count, int j0, int w,
+int launch_householder_panel(float *A, long long strideA, int n, int ld, int count, int j0, int w,
                              float *V, long long strideV, float *T, long long strideT, cudaStream_t s,
-                             int prev_w, const float *Tprev, int block_end) {
-    if (n <= 0 || count < 0 || j0 < 0 || j0 >= n || w <= 0 || w > kPanel || j0 + w > n) return record(QT_ERR_ARG);
+                             int prev_w, const float *Tprev, int block_end,
+                             void *planes_hi, void *planes_lo, long long ldp, long long strideP, int plane_col, int rows_above, int plane_exp) {
+    const PanelPlanes planes{static_cast<__half *>(planes_hi), static_cast<__half *>(planes_lo), ldp, strideP, plane_col, rows_above,
+                             ldexpf(1.0f, plane_exp)};
+    if (ld < n || n <= 0 || count < 0 || j0 < 0 || j0 >= n || w <= 0 || w > kPanel || j0 + w > n) return record(QT_ERR_ARG);
     if (!A || !V || !T) return record(QT_ERR_ARG);
     if (prev_w < 0 || prev_w > kPanel || prev_w > j0) return record(QT_ERR_ARG);
     if (prev_w > 0 && (!Tprev || block_end < j0 + w || block_end > n || block_end - j0 > 4 * kPanel)) return record(QT_ERR_ARG);
@@ -606,13 +629,13 @@ int launch_householder_panel(float *A, long long strideA, int n, int count, int 
     if (count > 65535) return record(QT_ERR_UNSUPPORTED);
     const int rows_per_lane = (n - j0 + 31) / 32;
     if (rows_per_lane > kMaxRowsPerLane) return record(QT_ERR_UNSUPPORTED);
-#define QT_PANEL(R, S) return launch_panel_rpl<R, S>(A, strideA, n, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end)
+#define QT_PANEL(R, S) return launch_panel_rpl<R, S>(A, strideA, n, ld, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end, planes)
     if (rows_per_lane <= 6) QT_PANEL(6, 0);
     if (rows_per_lane <= 12) QT_PANEL(12, 0);
     if (rows_per_lane <= 20) QT_PANEL(20, 0);
     if (g_panel_pairs && rows_per_lane > 20) {
-        if (rows_per_lane <= 28) return launch_panel_pairs<28>(A, strideA, n, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end);
-        return launch_panel_pairs<38>(A, strideA, n, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end);
+        if (rows_per_lane <= 28) return launch_panel_pairs<28>(A, strideA, n, ld, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end, planes);
+        return launch_panel_pairs<38>(A, strideA, n, ld, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end, planes);
     }
     if (rows_per_lane <= 28) QT_PANEL(24, 4);
     QT_PANEL(24, 14);
@@ -629,7 +652,8 @@ static constexpr int kMergeMax = 128;
 __global__ void __launch_bounds__(1024)
 k_merge_t(const float *__restrict__ Gbase, long long ldg, long long strideG,
           const float *__restrict__ Tp_base, long long strideTp, int wo,
-          float *__restrict__ Tbase, long long strideT) {
+          float *__restrict__ Tbase, long long strideT,
+          __half *__restrict__ hi, __half *__restrict__ lo, long long ldp, long long strideP, int *__restrict__ exp_out, int target) {
     extern __shared__ float merge_sm[];
     float (*Ts)[kMergeMax + 1] = reinterpret_cast<float (*)[kMergeMax + 1]>(merge_sm);
     float (*M1)[kPanel + 1] = reinterpret_cast<float (*)[kPanel + 1]>(merge_sm + kMergeMax * (kMergeMax + 1));
@@ -671,14 +695,39 @@ k_merge_t(const float *__restrict__ Gbase, long long ldg, long long strideG,
         }
         __syncthreads();
     }
+    if (Tbase)
+        for (int i = ty; i < wo; i += 32)
+            for (int j = tx; j < wo; j += 32) T[(long long)i * wo + j] = Ts[i][j];
+    if (!hi) return;
+    // scaled fp16 planes of T (the operand of the products that follow), exponent from the largest magnitude
+    float am = 0.0f;
     for (int i = ty; i < wo; i += 32)
-        for (int j = tx; j < wo; j += 32) T[(long long)i * wo + j] = Ts[i][j];
+        for (int j = tx; j < wo; j += 32) am = fmaxf(am, fabsf(Ts[i][j]));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, off));
+    if (tx == 0) M1[0][ty] = am;
+    __syncthreads();
+    am = M1[0][tx];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, off));
+    const int e = exponent_for(am, target);
+    if (threadIdx.x == 0) exp_out[blockIdx.x] = e;
+    const float two_e = exp2f((float)e);
+    hi += (long long)blockIdx.x * strideP;
+    lo += (long long)blockIdx.x * strideP;
+    for (int i = ty; i < wo; i += 32)
+        for (int j = tx; j < wo; j += 32) {
+            const float x = fminf(fmaxf(Ts[i][j] * two_e, -65000.0f), 65000.0f);
+            const __half h = __float2half_rn(x);
+            hi[(long long)i * ldp + j] = h;
+            lo[(long long)i * ldp + j] = __float2half_rn(x - __half2float(h));
+        }
 }
 
 int launch_merge_t(const float *G, long long ldg, long long strideG, const float *Tp, long long strideTp, int wo, int count,
-                   float *T, long long strideT, cudaStream_t s) {
+                   float *T, long long strideT, cudaStream_t s, void *hi, void *lo, long long ldp, long long strideP, int *exp_out, int target) {
     if (wo <= 0 || wo > kMergeMax || count < 0 || ldg < wo) return record(QT_ERR_ARG);
-    if (!G || !Tp || !T) return record(QT_ERR_ARG);
+    if (!G || !Tp || (!T && !hi) || (hi && (!lo || !exp_out || ldp < wo))) return record(QT_ERR_ARG);
     if (count == 0) return record(QT_OK);
     constexpr size_t smem = sizeof(float) * (2 * kMergeMax * (kMergeMax + 1) + 96 * (kPanel + 1) + kPanel * (kPanel + 1));
     static PerDeviceOnce attr_set;
@@ -688,7 +737,8 @@ int launch_merge_t(const float *G, long long ldg, long long strideG, const float
             return record(QT_ERR_LAUNCH);
         attr_set.mark(dev);
     }
-    k_merge_t<<<count, 1024, smem, s>>>(G, ldg, strideG, Tp, strideTp, wo, T, strideT);
+    k_merge_t<<<count, 1024, smem, s>>>(G, ldg, strideG, Tp, strideTp, wo, T, strideT, static_cast<__half *>(hi), static_cast<__half *>(lo), ldp,
+                                        strideP, exp_out, target);
     count_launch(1);
     return check_launch();
 }

@@ -50,9 +50,13 @@ struct DequantArgs {
     void *out; int out_dtype; long long stride_out;         // elements
 };
 
-int read_apply_error(bool clear);  // error word of the kernels in apply_kernels.cu
+int launch_grad_planes(const void *stat_items, int n_stat, const void *split_items, int n_split, const long long *grads, float *part_amax,
+                       float *part_ss, int *gexp, int target, void *plane_base, cudaStream_t stream);
+int read_apply_error(bool clear);    // error words of the kernels in apply_kernels.cu and refresh.cu
+int read_refresh_error(bool clear);
 int launch_merge_t(const float *G, long long ldg, long long strideG, const float *Tp, long long strideTp, int wo, int count,
-                   float *T, long long strideT, cudaStream_t stream);
+                   float *T, long long strideT, cudaStream_t stream, void *hi = nullptr, void *lo = nullptr, long long ldp = 0,
+                   long long strideP = 0, int *exp_out = nullptr, int target = 0);
 int launch_quantize(const QuantArgs &a, cudaStream_t stream);
 int launch_dequantize(const DequantArgs &a, cudaStream_t stream);
 // a.out / a.out_dtype / a.stride_out are ignored: output goes to the bf16 planes hi, lo
@@ -65,8 +69,11 @@ int launch_state_exponents(const float *absmax, long long stride_absmax, int n_a
 int launch_selftest_division(unsigned long long seed, unsigned long long pairs, unsigned long long *mismatches_dev,
                              cudaStream_t stream);
 void set_panel_pairs(int on);
-int launch_householder_panel(float *A, long long strideA, int n, int count, int j0, int w,
+int launch_householder_panel(float *A, long long strideA, int n, int ld, int count, int j0, int w,
                              float *V, long long strideV, float *T, long long strideT, cudaStream_t stream,
-                             int prev_w = 0, const float *Tprev = nullptr, int block_end = 0);
+                             int prev_w = 0, const float *Tprev = nullptr, int block_end = 0,
+                             // scaled fp16 planes of V (see qr_kernels.cu); null: none
+                             void *planes_hi = nullptr, void *planes_lo = nullptr, long long ldp = 0, long long strideP = 0,
+                             int plane_col = 0, int rows_above = 0, int plane_exp = 0);
 
 }  // namespace qt

@@ -317,7 +317,6 @@ class ApplyPlan:
             self._tensors[i] = (0, 0, 0, d_base + 4 * d_off[i] if i in widths else 0, n, i, flags, *g_range[i], r0, len(rr), 0)
         self._tensor_table = torch.zeros(self._tensors.nbytes, dtype=torch.uint8, device=dev)
         self._state_ptrs = None
-        self.grads = PointerTable(len(params), dev)
         d = self.desc = Desc()
         d.stat_items, d.n_stat_items = up(table(stat)), len(stat)
         d.waves, d.n_waves = ct.addressof(self.waves), len(wave_tables)

@@ -19,8 +19,10 @@ import qtensor.functional as F
 from qtensor.utils import QTensorDiagReal, QTensorSVDFast
 from optimizers import _apply
 from optimizers import _engine as E
+from optimizers import _refresh
 
 FUSED_TAIL = True              # AdamW tail as one multi-tensor launch of the library (CUDA fp32 parameters)
+PLANNED_REFRESH = True         # eigen-factor statistics and roots of an order class as one host call (optimizers/_refresh.py)
 PLANNED_APPLY = True           # directions, grafting and tail of an unsharded step through a plan (optimizers/_apply.py)
 
 CODE = 'linear-2'
@@ -427,23 +429,90 @@ class _ShampooBase(optim.Optimizer):
     def _refresh(self, group, params):
         """Counts the step and refreshes statistics and inverse roots of `params` where their intervals fire."""
         t1, t2 = group['stat_compute_steps'], group['prec_compute_steps']
-        stat_items, root_items = [], []
+        states = [self.state[p] for p in params]
+        for st in states:
+            st['step'] += 1
+        step = states[0]['step']
+        one_step = all([st['step'] == step for st in states])
+        if one_step and step % t1 and step % t2:
+            return
         w1 = group['stat_decay']
         w2 = 1.0 if w1 == 1.0 else 1.0 - w1
-        for p in params:
-            state = self.state[p]
-            state['step'] += 1
-            if state['step'] % t1 == 0:
-                pre = state['preconditioner']
-                if pre.statistics:
+        eps, mode = group['matrix_eps'], group.get('inv_root_mode', 0)
+        for st in states:
+            if st['step'] % t2 == 0:
+                st['preconditioner']._active = True
+        planned, rest = {}, True
+        if one_step:
+            plan, table = self._refresh_plan_for(group, params, step)
+            if plan is not None:
+                stat, root = step % t1 == 0, step % t2 == 0
+                for cls in plan.batches:
+                    planned[cls] = lambda cls=cls: plan.run(cls, table, stat, root, w1, w2, eps)
+                rest = plan.rest
+        stat_items, root_items = [], []
+        if rest:
+            for p, st in zip(params, states):
+                pre = st['preconditioner']
+                if st['step'] % t1 == 0 and pre.statistics:
                     stat_items += pre.statistics_items(p.grad.data)
-            if state['step'] % t2 == 0:
-                pre = state['preconditioner']
-                root_items += pre._slots
-                pre._active = True
-        if stat_items or root_items:
-            E.refresh(stat_items, root_items, w1, w2, group['matrix_eps'], group.get('inv_root_mode', 0),
-                      exact=(group.get('inv_root_mode', 0) != 0))
+                if st['step'] % t2 == 0:
+                    root_items += pre._slots
+        if stat_items or root_items or planned:
+            E.refresh(stat_items, root_items, w1, w2, eps, mode, exact=(mode != 0), planned=planned)
+
+    def _known(self, params):
+        """What is remembered for a list of parameters: plans and the device table of their gradients' addresses."""
+        ids = tuple(map(id, params))
+        known = self._apply_plans.get(ids)
+        if known is None:
+            if len(self._apply_plans) >= 4:                   # bounded: plans own workspaces
+                self._apply_plans.clear()
+            known = self._apply_plans[ids] = {"params": params, "states": [self.state[p] for p in params], "plans": {},
+                                              "refresh": None, "grads": None, "table": (-1, None)}
+        return known
+
+    def _gradient_table(self, known, params, step):
+        """Device table of this step's gradients, or None if one of them is not dense fp32 on the parameters' device."""
+        table = self.__dict__.get("_grad_table")              # a captured step reads its own gradient buffers
+        if table is not None:
+            return table
+        if known["table"][0] == step:
+            return known["table"][1]
+        dev = params[0].device
+        ptrs = []
+        for p in params:
+            g = p.grad
+            if g.dtype != torch.float32 or not g.is_contiguous() or g.device != dev:
+                return None
+            ptrs.append(g.data_ptr())
+        if known["grads"] is None:
+            known["grads"] = _apply.PointerTable(len(params), dev)
+        if torch.cuda.is_current_stream_capturing() and ptrs != known["grads"].ptrs:
+            return None
+        known["grads"].set(ptrs)
+        known["table"] = (step, known["grads"].dev)
+        return known["grads"].dev
+
+    def _plannable(self, group, params):
+        return (self._world == 1 and F.lib is not None and not E.REFERENCE_DIAGREAL_NONE and E.USE_TENSOR_CORES
+                and group['prec_bits'] in (4, 8) and params[0].device.type == "cuda")
+
+    def _refresh_plan_for(self, group, params, step):
+        """(plan, gradient table) of the refresh, or (None, None) where the general engine has to take all of it."""
+        if not PLANNED_REFRESH or not self._plannable(group, params):
+            return None, None
+        known = self._known(params)
+        if known["refresh"] is None:
+            dev = params[0].device
+            if torch.cuda.is_current_stream_capturing() or any(p.device != dev or p.dtype != torch.float32 for p in params):
+                return None, None
+            with torch.cuda.device(dev):
+                known["refresh"] = _refresh.RefreshPlan(params, known["states"], group.get('inv_root_mode', 0))
+        table = self._gradient_table(known, params, step)
+        if table is None:
+            return None, None
+        return known["refresh"], table
 
     # ---- planned application (optimizers/_apply.py) ------------------------------------------
     _plan_kind, _plan_moments = None, ()                      # set by the SGD / AdamW variants
@@ -451,15 +520,9 @@ class _ShampooBase(optim.Optimizer):
     def _plan_for(self, group, params, step):
         """The plan for these parameters at this step, or None where the general path has to take it: sharded or
         CPU runs, 16/32-bit preconditioners, gradients that are not dense fp32, steps that differ between parameters."""
-        if (not PLANNED_APPLY or self._plan_kind is None or self._world > 1 or F.lib is None or E.REFERENCE_DIAGREAL_NONE
-                or not E.USE_TENSOR_CORES or group['prec_bits'] not in (4, 8) or not FUSED_TAIL):
+        if not PLANNED_APPLY or self._plan_kind is None or not FUSED_TAIL or not self._plannable(group, params):
             return None
-        ids = tuple(map(id, params))
-        known = self._apply_plans.get(ids)
-        if known is None:
-            if len(self._apply_plans) >= 4:                   # bounded: plans own workspaces
-                self._apply_plans.clear()
-            known = self._apply_plans[ids] = {"params": params, "states": [self.state[p] for p in params], "plans": {}}
+        known = self._known(params)
         states = known["states"]
         for st in states:
             if st['step'] != step:
@@ -468,9 +531,9 @@ class _ShampooBase(optim.Optimizer):
         plan = known["plans"].get(grafted)
         if plan is None:
             dev = params[0].device
-            if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
+            if torch.cuda.is_current_stream_capturing():
                 return None
-            if dev.type != "cuda" or any(p.device != dev or p.dtype != torch.float32 for p in params):
+            if any(p.device != dev or p.dtype != torch.float32 for p in params):
                 plan = False
             else:
                 if len(known["plans"]) >= 2:
@@ -491,18 +554,9 @@ class _ShampooBase(optim.Optimizer):
         plan = self._plan_for(group, params, step)
         if plan is None:
             return False
-        table = self.__dict__.get("_grad_table")              # a captured step reads its own gradient buffers
+        table = self._gradient_table(self._known(params), params, step)
         if table is None:
-            ptrs = []
-            for p in params:
-                g = p.grad
-                if g.dtype != torch.float32 or not g.is_contiguous():
-                    return False
-                ptrs.append(g.data_ptr())
-            if torch.cuda.is_current_stream_capturing() and ptrs != plan.grads.ptrs:
-                return False
-            plan.grads.set(ptrs)
-            table = plan.grads.dev
+            return False
         with F._on_device(table):
             plan.run(table, F._stream(table), scalars, **self._plan_hyper(group, step))
         return True
@@ -660,6 +714,7 @@ class _ShampooBase(optim.Optimizer):
             if fires_root:
                 st['preconditioner']._active = True
         self._plan_for(group, params, step)
+        self._refresh_plan_for(group, params, step)
         for st, (n, act) in zip(states, book):
             st['step'], st['preconditioner']._active = n, act
 

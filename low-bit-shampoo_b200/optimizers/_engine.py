@@ -593,9 +593,14 @@ def compute_preconditioners(items, eps, inv_root_mode, exponent=4):
         _class_roots(cls, slots, eps, inv_root_mode, exponent, starts)
 
 
-def refresh(stat_items, root_items, w1, w2, eps, inv_root_mode, exact=False, exponent=4):
+def refresh(stat_items, root_items, w1, w2, eps, inv_root_mode, exact=False, exponent=4, planned=None):
     """add_statistics followed by compute_preconditioners, pipelined per order class: a class
-    starts its inverse roots as soon as its own statistics are done, on the same stream."""
+    starts its inverse roots as soon as its own statistics are done, on the same stream.
+    `planned`: {class: callable} - classes whose whole refresh is that call (their items are ignored)."""
+    planned = planned or {}
+    if planned:
+        stat_items = [e for e in stat_items if e[0] not in planned]
+        root_items = [e for e in root_items if e[0] not in planned]
     starts = _newton_starts(root_items, inv_root_mode)
     stats, roots = defaultdict(list), defaultdict(list)
     for cls, slot, g, axis in stat_items:
@@ -603,7 +608,12 @@ def refresh(stat_items, root_items, w1, w2, eps, inv_root_mode, exact=False, exp
     for cls, slot in root_items:
         roots[cls].append(slot)
     merged = {cls: (stats.get(cls, []), roots.get(cls, [])) for cls in list(stats) + [c for c in roots if c not in stats]}
-    for cls, (entries, slots) in _over_units(_split_units(merged)):
+    units = _split_units(merged) + [(float(cls.n) ** 3 * cls.count, cls, None) for cls in planned]
+    for cls, item in _over_units(units):
+        if item is None:
+            planned[cls]()
+            continue
+        entries, slots = item
         if entries:
             _class_statistics(cls, entries, w1, w2, eps, exact)
         if slots:
