@@ -329,6 +329,8 @@ typedef struct qt_gemm_desc {
                      * the whole product); 0: one CTA per SM */
     int c_follows_d; /* != 0: the C operand of matrix b is entry d_slot[b] of its array, like the outputs
                       * (C == D then updates selected entries of an array in place) */
+    int sym;         /* != 0: the result is symmetric (M == N): tiles on and above the diagonal are computed and mirrored
+                      * (not with 4-bit state) */
 } qt_gemm_desc;
 int qt_gemm_ex(const qt_gemm_desc *desc, void *stream);
 

@@ -17,9 +17,13 @@
 // on the three-plane tcgen05 kernel (fp32-level accuracy), each epilogue writing the planes the
 // next product reads; the epilogue of T^p M also writes the next T and reduces max |M' - I|.
 #include "qt_common.cuh"
+#include <cooperative_groups.h>
+#include <cstring>
 #include <math_constants.h>
 
 namespace qt {
+
+namespace cg = cooperative_groups;
 
 __device__ __forceinline__ float warp_sum_f(float v) {
 #pragma unroll
@@ -40,46 +44,57 @@ __device__ __forceinline__ double block_sum(double v, double *scratch /*[32]*/) 
     return t;
 }
 
-// One CTA per matrix.  Power iteration exactly as PowerIter states it (normalise, multiply,
+// One cluster per matrix.  Power iteration exactly as PowerIter states it (normalise, multiply,
 // Rayleigh quotient, stop when it moves by <= tol or after max_iters), then - if ridge_eps >= 0 -
 // the ridge ridge_eps * lambda_max is added to the diagonal IN PLACE (the reference mutates its
 // argument too, matrix_functions.py:112) and the Frobenius norm of the result is written.
+// Bound by what an SM draws from L2 in each of the ten dependent sweeps (one CTA per matrix: 50 us per sweep at order
+// 1200), so the rows are spread over the CTAs of a cluster; every CTA holds the whole vector and writes its part of the
+// product into the shared memory of all of them.  Order 1200 alone on the chip: 510 -> 120 us with eight CTAs.
 __global__ void __launch_bounds__(1024, 1)
 k_power_iter(float *__restrict__ Gbase, long long strideG, int n, const float *__restrict__ v0, float tol, int max_iters,
              float ridge_eps, float *__restrict__ max_ev, float *__restrict__ fro, int *__restrict__ iters_out,
              float *__restrict__ vec_out) {
     extern __shared__ float pw_sm[];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     float *v = pw_sm, *y = pw_sm + n;
-    __shared__ double red[32];
-    float *G = Gbase + (long long)blockIdx.x * strideG;
+    __shared__ double red[32], part[8];
+    const int mat = blockIdx.x / cs;
+    float *G = Gbase + (long long)mat * strideG;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-    for (int i = tid; i < n; i += blockDim.x) v[i] = v0[(long long)blockIdx.x * n + i];
+    const int row0 = rank * warps + warp, row_step = warps * cs;
+    float *y_peer = lane < cs ? cluster.map_shared_rank(y, lane) : nullptr;
+    for (int i = tid; i < n; i += blockDim.x) v[i] = v0[(long long)mat * n + i];
     __syncthreads();
     const bool vec = (n & 3) == 0 && ((reinterpret_cast<uintptr_t>(G) & 15) == 0);
     float sval = 0.0f, err = 1.0f;
     int it = 0;
-    while (err > tol && it < max_iters) {
+    while (err > tol && it < max_iters) {                    // the same decisions in every CTA of the cluster
         double ss = 0.0;
         for (int i = tid; i < n; i += blockDim.x) ss += (double)v[i] * (double)v[i];
         const float nrm = (float)sqrt(block_sum(ss, red));
         for (int i = tid; i < n; i += blockDim.x) v[i] = v[i] / nrm;
-        __syncthreads();
-        for (int r = warp; r < n; r += warps) {
+        cluster.sync();                                       // v is complete; no CTA still reads y
+        for (int r = row0; r < n; r += row_step) {
             const float *row = G + (long long)r * n;
             float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
             if (vec) {
+#pragma unroll 4
                 for (int c = lane * 4; c < n; c += 128) {
                     const float4 g = *reinterpret_cast<const float4 *>(row + c);
-                    a0 = fmaf(g.x, v[c], a0); a1 = fmaf(g.y, v[c + 1], a1);
-                    a2 = fmaf(g.z, v[c + 2], a2); a3 = fmaf(g.w, v[c + 3], a3);
+                    const float4 x = *reinterpret_cast<const float4 *>(v + c);
+                    a0 = fmaf(g.x, x.x, a0); a1 = fmaf(g.y, x.y, a1);
+                    a2 = fmaf(g.z, x.z, a2); a3 = fmaf(g.w, x.w, a3);
                 }
             } else {
+#pragma unroll 4
                 for (int c = lane; c < n; c += 32) a0 = fmaf(row[c], v[c], a0);
             }
             const float d = warp_sum_f((a0 + a1) + (a2 + a3));
-            if (lane == 0) y[r] = d;
+            if (y_peer) y_peer[r] = d;
         }
-        __syncthreads();
+        cluster.sync();
         double dot = 0.0;
         for (int i = tid; i < n; i += blockDim.x) dot += (double)v[i] * (double)y[i];
         const float s = (float)block_sum(dot, red);
@@ -89,25 +104,33 @@ k_power_iter(float *__restrict__ Gbase, long long strideG, int n, const float *_
         __syncthreads();
         ++it;
     }
-    if (tid == 0) {
-        max_ev[blockIdx.x] = sval;
-        if (iters_out) iters_out[blockIdx.x] = it;
+    if (rank == 0 && tid == 0) {
+        max_ev[mat] = sval;
+        if (iters_out) iters_out[mat] = it;
     }
-    if (vec_out)
-        for (int i = tid; i < n; i += blockDim.x) vec_out[(long long)blockIdx.x * n + i] = v[i];
-    if (ridge_eps < 0.0f || fro == nullptr) return;
-    const float ridge = ridge_eps * sval;
-    for (int r = tid; r < n; r += blockDim.x) G[(long long)r * n + r] += ridge;
-    __syncthreads();
-    double sq = 0.0;
-    for (int r = warp; r < n; r += warps) {
-        const float *row = G + (long long)r * n;
-        float a0 = 0.0f;
-        for (int c = lane; c < n; c += 32) a0 = fmaf(row[c], row[c], a0);
-        sq += (double)a0;
+    if (rank == 0 && vec_out)
+        for (int i = tid; i < n; i += blockDim.x) vec_out[(long long)mat * n + i] = v[i];
+    if (ridge_eps >= 0.0f && fro != nullptr) {
+        const float ridge = ridge_eps * sval;
+        double sq = 0.0;
+        for (int r = row0; r < n; r += row_step) {
+            float *row = G + (long long)r * n;
+            if (lane == 0) row[r] += ridge;
+            __syncwarp();
+            float a0 = 0.0f;
+            for (int c = lane; c < n; c += 32) a0 = fmaf(row[c], row[c], a0);
+            sq += (double)a0;
+        }
+        const double mine = block_sum(sq, red);
+        if (tid == 0) *cluster.map_shared_rank(part + rank, 0) = mine;
+        cluster.sync();
+        if (rank == 0 && tid == 0) {
+            double total = 0.0;
+            for (int i = 0; i < cs; ++i) total += part[i];
+            fro[mat] = (float)sqrt(total);
+        }
     }
-    const double total = block_sum(sq, red);
-    if (tid == 0) fro[blockIdx.x] = (float)sqrt(total);
+    cluster.sync();                                           // no CTA leaves while another may still write to it
 }
 
 __device__ __forceinline__ void split3_store(float x, __nv_bfloat16 *hi, __nv_bfloat16 *mid, __nv_bfloat16 *lo, long long o) {
@@ -207,7 +230,24 @@ int launch_power_iter(float *G, long long strideG, int n, int batch, const float
             return record(QT_ERR_LAUNCH);
         attr.mark(dev);
     }
-    k_power_iter<<<batch, 1024, smem, s>>>(G, strideG, n, v0, tol, max_iters, ridge_eps, max_ev, fro, iters, vec_out);
+    // as many CTAs per matrix as keep every SM at one CTA (eight is the portable limit); a matrix below 64 rows gains nothing
+    int cs = 1;
+    while (cs < 8 && 2 * cs * batch <= device_sm_count() && n >= 64 * cs) cs *= 2;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)(batch * cs), 1, 1);
+    cfg.blockDim = dim3(1024, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_power_iter, G, strideG, n, v0, tol, max_iters, ridge_eps, max_ev, fro, iters, vec_out) != cudaSuccess) {
+        cudaGetLastError();
+        return record(QT_ERR_LAUNCH);
+    }
     count_launch(1);
     return check_launch();
 }

@@ -342,3 +342,27 @@ def test_column_dot_is_accurate_and_independent_of_the_batch(native_lib):
         assert float((full.double() - ref).abs().max() / ref.abs().max()) < 1e-6
         part = E.column_dot(A[:small].contiguous(), B[:small].contiguous())
         assert torch.equal(full[:small], part)
+
+
+@pytest.mark.parametrize("planes", [2, 3])
+@pytest.mark.parametrize("n,k", [(64, 40), (128, 128), (130, 65), (257, 300), (400, 16)])
+def test_symmetric_product_equals_the_full_product(native_lib, n, k, planes):
+    """Half of the tiles, mirrored: fp32 result with a C operand through a slot list, and plane outputs, at tile edges."""
+    from optimizers import _gemm
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    G = torch.randn(3, n, k, device="cuda", generator=g)
+    C0 = torch.randn(5, n, n, device="cuda", generator=g)
+    C0 = C0 + C0.transpose(1, 2)
+    P = _gemm.split(G) if planes == 2 else _gemm.split3(G)
+    sel = torch.tensor([4, 0, 2], dtype=torch.int32, device="cuda")
+    out = {}
+    for sym in (False, True):
+        C = C0.clone()
+        _gemm.gemm_ex(P, P, trans_b=True, alpha=0.3, beta=0.7, C=C, D=C, d_slot=sel, c_follows_d=True, batch=3, sym=sym)
+        Q = _gemm.Planes(3, n, n, "cuda", planes=planes, f16=planes == 2)
+        Q.exp0 = 4 if planes == 2 else 0
+        _gemm.gemm_ex(P, P, trans_b=True, P=Q, out_exp0=4, sym=sym)
+        out[sym] = C, Q.to_float()
+    for x, y in zip(out[True], out[False]):
+        assert float((x - y).abs().max()) <= 3e-6 * float(y.abs().max())
+    assert torch.equal(out[True][0][[1, 3]], C0[[1, 3]])
