@@ -36,8 +36,8 @@ __device__ __forceinline__ void store_panel_planes(const PanelPlanes &pp, const 
 static constexpr int kPanel = 32;
 static constexpr int kQrThreads = 1024;                    // one warp per panel column
 static constexpr int kMaxRowsPerLane = 38;                 // panel rows <= 32 * 38 = 1216
-static int g_panel_pairs = 1;                              // measurement hook: 0 = one column per warp at every height
-void set_panel_pairs(int on) { g_panel_pairs = on; }
+static int g_panel_blocked = 1;                            // test hook: 0 = the kernel with one column per warp
+void set_panel_blocked(int on) { g_panel_blocked = on; }
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -45,7 +45,8 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// Register-resident panel: warp c owns column c, lane l holds rows l, l+32, ... of it for the
+// The kernel with one column per warp, kept as the independent form that tests compare the panel kernel with
+// (qt_panel_force_form).  Register-resident panel: warp c owns column c, lane l holds rows l, l+32, ... of it for the
 // whole factorisation: the first RPL of them in registers, RS more (tall panels only) in the
 // column's slots of the shared staging buffer, so that the register budget of a 1024-thread CTA
 // (64 per thread) is never exceeded.  Per column step the pivot warp builds its Householder
@@ -321,254 +322,483 @@ k_householder_panel(float *__restrict__ Abase, long long strideA, int n, int ld,
 }
 
 
-// Tall panels (more than 640 rows): two columns per warp, 16 warps.  With one column per warp every
-// warp reads the whole published Householder vector twice per step and the tall variants also keep
-// part of their column in shared memory (64 registers per thread at 1024 threads); here a warp
-// reads the vector once for both of its columns and a thread's 2 x RT elements all live in
-// registers (128 per thread at 512 threads): a third of the shared-memory traffic per step.
-// Warp w owns columns 2w, 2w+1 and rows 2w, 2w+1 of T.  Same conventions, same fused update of the
-// previous panel, same outputs as k_householder_panel.
+// ------------------------------------------------------------------------------------
+// The panel kernel.  16 warps, warp w owns columns 2w and 2w+1, lane l rows l, l+32, .. of them, in registers (2 RT
+// values per thread).  The 32 columns are factored in four sub-panels of eight.  Inside a sub-panel only the four warps
+// that own its columns take part.  Per column step the pivot column x is published as it is, one barrier of 128 threads,
+// and every warp reduces ||x||^2 together with the products of x and its own columns: one round of shuffles, no pivot
+// phase that the others wait for (v = (1, x / (alpha - beta)) is a scaling that can follow).  A finished sub-panel is
+// applied to the columns on its right as a block of eight: one pass over the rows for eight products per column, one
+// combined reduction, a forward substitution (z_j = tau_j (w_j - sum_i<j (v_i . v_j) z_i), no triangular factor needed),
+// one pass for the update - while the next sub-panel's warps, which have their own pass first, already go on factoring
+// and finished columns take their products with the new vectors for the triangular factor.
+//
+// What bounds it is the dependent chain of 32 column steps (700 clocks each on short panels: barrier, reduction, square
+// root, reciprocals).  With every warp multiplying and updating its columns in every step, and a separate pivot phase,
+// a step of a tall panel took 3700 clocks.  Per launch, without / with the fused update below: 968 rows 72 / 101 -> 42 /
+// 62 us, 480 rows 42 / 60 -> 28 / 41, 96 rows 25 / 32 -> 19 / 27.
+//
+// Fused form (prev_w > 0): the block reflector of the previous panel is applied first, C <- (I - Vp Tp^T Vp^T) C on the
+// window rows j0 - prev_w .. n-1; CTA (matrix, chunk) takes 32 columns, chunk 0 is the panel itself.  Both
+// products run on mma.sync (m16n8k8, tf32): every fp32 operand is split into two tf32 values, three products each,
+// which keeps 2^-23 relative; at 32 columns the tile is far too small for tcgen05 and the operands come straight from
+// L2 (Vp) and the shared image (C).
+// ------------------------------------------------------------------------------------
+static constexpr int kPw = 16, kPt = kPw * 32;            // warps and threads of a panel CTA
+static constexpr int kPp = 33;                            // row pitch of the shared image: columns and 32-row groups conflict-free
+
+// x = hi + lo to 2^-23: both rounded to tf32's 11 significant bits (half away from zero); the tensor core ignores the low
+// 13 bits of an operand, so lo needs no mask.
+__device__ __forceinline__ void tf32_split(float x, unsigned &hi, unsigned &lo) {
+    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
+}
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// Sum of 16 values over the lanes of a warp; every lane receives all of them.
+__device__ __forceinline__ void warp_sum16(float (&v)[16], int lane) {
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = v[i];
+#pragma unroll
+    for (int h = 8; h >= 1; h >>= 1) {                       // lane bit 2h decides which half of the values it keeps
+        const bool upper = (lane & (2 * h)) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float keep = upper ? x[i + h] : x[i], give = upper ? x[i] : x[i + h];
+            x[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+        }
+    }
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __shfl_sync(0xffffffffu, x[0], 2 * i);   // value i sits in lanes 2i, 2i+1
+}
+
+// Products of a warp's two columns with eight vectors of the shared image (columns s0 .. s0+7; Pl: this lane's rows).
 template <int RT>
-__global__ void __launch_bounds__(512, 1)
-k_householder_panel_pairs(float *__restrict__ Abase, long long strideA, int n, int ld, int j0, int w,
-                          float *__restrict__ Vbase, long long strideV, float *__restrict__ Tbase, long long strideT,
-                          int prev_w, const float *__restrict__ Tprev_base, int block_end, const PanelPlanes planes) {
-    constexpr int NW = 16, NT = NW * 32;
+__device__ __forceinline__ void dot8(const float *Pl, int s0, const float (&colA)[RT], const float (&colB)[RT], float (&z)[16], int lane) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) z[j] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < RT; ++k)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float v = Pl[32 * k * kPp + s0 + j];
+            z[j] = fmaf(v, colA[k], z[j]);
+            z[8 + j] = fmaf(v, colB[k], z[8 + j]);
+        }
+    warp_sum16(z, lane);
+}
+
+template <int RT>
+__global__ void __launch_bounds__(kPt, 1)
+k_panel(float *__restrict__ Abase, long long strideA, int n, int ld, int j0, int w, float *__restrict__ Vbase, long long strideV,
+        float *__restrict__ Tbase, long long strideT, int prev_w, const float *__restrict__ Tprev_base, int block_end, const PanelPlanes planes) {
     extern __shared__ float sm[];
     const int m = n - j0;
-    float *Pall = sm;                                      // [kPanel + m][33]
-    float *P = Pall + kPanel * 33;
-    float *vb = Pall + (((kPanel + m) * 33 + 31) & ~31);   // [2][RT * 32] published Householder vector
-    float *G = vb + 2 * RT * 32;                           // [32][33]
-    float *Ts = G + kPanel * (kPanel + 1);                 // [32][33]
-    float *tau = Ts + kPanel * (kPanel + 1);               // [32]
-    float *Vs = tau + kPanel;                              // [256][36]
-    float *Tp = Vs + 256 * 36;                             // [32][33]
-    float *zs = Tp + kPanel * (kPanel + 1);                // [32][33]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int chunk = blockIdx.y;
+    float *Pall = sm;                                      // [32 + 32 RT + 32][33]: window rows above the panel, panel rows, zeros
+    float *P = Pall + kPanel * kPp;
+    float *part = Pall + (32 * RT + 64) * kPp;             // [8][32][33] partial sums; later the published pivot columns
+    float *G = part + 8 * 32 * 33;                         // [32][33] v_i . v_j, i < j
+    float *Ts = G + 32 * 33;                               // [32][33]
+    float *Tp = Ts + 32 * 33, *Wm = Tp + 32 * 33, *zs = Wm + 32 * 33;
+    float *tau = zs + 32 * 33;                             // [32]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, chunk = blockIdx.y;
+    const int g = lane >> 2, tig = lane & 3;               // fragment coordinates of mma.m16n8k8
     float *Amat = Abase + (long long)blockIdx.x * strideA;
-    const float *A = Amat + (long long)j0 * ld + j0;
+    float *V = Vbase + (long long)blockIdx.x * strideV;
 
+    const int r0 = j0 - prev_w, mu = m + prev_w;           // window: first row, rows
+    const int c0 = j0 + kPanel * chunk, wc = min(kPanel, prev_w > 0 ? block_end - c0 : w);
+    float *C = P - prev_w * kPp;                           // window row 0
+    float *Cg = Amat + (long long)r0 * ld + c0;
+    if (wc == kPanel && (ld & 3) == 0 && (strideA & 3) == 0 && (reinterpret_cast<uintptr_t>(Abase) & 15) == 0) {
+        // a warp takes four rows at a time, 16 bytes per lane; the four stores of a lane meet 32 different banks
+#pragma unroll 8
+        for (int r = 4 * warp + (lane >> 3); r < mu; r += 4 * kPw) {
+            const float4 x = *reinterpret_cast<const float4 *>(Cg + (long long)r * ld + 4 * (lane & 7));
+            float *dst = C + r * kPp + 4 * (lane & 7);
+            dst[0] = x.x; dst[1] = x.y; dst[2] = x.z; dst[3] = x.w;
+        }
+    } else {
+#pragma unroll 8
+        for (int r = warp; r < mu; r += kPw) C[r * kPp + lane] = lane < wc ? Cg[(long long)r * ld + lane] : 0.0f;
+    }
+    for (int r = mu + warp; r < 32 * RT + 32 + prev_w; r += kPw) C[r * kPp + lane] = 0.0f;   // up to the end of the image
     if (prev_w > 0) {
-        // ---- apply the previous panel's block reflector to this CTA's column chunk
-        const int r0 = j0 - prev_w;                        // first row of the update window
-        const int mu = n - r0;                             // rows of the window
-        const int c0 = j0 + kPanel * chunk;                // first column of the chunk
-        const int wc = min(kPanel, block_end - c0);        // columns of the chunk
-        float *C = Pall + (kPanel - prev_w) * 33;          // window rows so that row prev_w of it is P's row 0
-        float *Cg = Amat + (long long)r0 * ld + c0;
-        const float *Vg = Vbase + (long long)blockIdx.x * strideV + (long long)r0 * ld + r0;
-        for (int r = warp; r < mu; r += NW) C[r * 33 + lane] = (lane < wc) ? Cg[(long long)r * ld + lane] : 0.0f;
-        for (int i = tid; i < kPanel * kPanel; i += NT) {
-            const int a = i / kPanel, b = i - a * kPanel;
-            Tp[a * (kPanel + 1) + b] = (a < prev_w && b < prev_w) ? Tprev_base[(long long)blockIdx.x * strideT + i] : 0.0f;
+        for (int i = tid; i < 32 * 32; i += kPt) {
+            const int a = i >> 5, b = i & 31;
+            Tp[a * 33 + b] = (a < prev_w && b < prev_w) ? Tprev_base[(long long)blockIdx.x * strideT + i] : 0.0f;
         }
-        // Vp is streamed through shared memory in slabs of kSlab window rows; the next slab is
-        // fetched into registers while the current one is being used, so the global-memory latency
-        // of the 2 * ceil(mu / kSlab) dependent slab loads is hidden behind the arithmetic.
-        // In both passes a lane works on COLUMN `lane` of the chunk and a warp on a subset of the rows,
-        // so a row of Vp is read as broadcast 128-bit loads and serves all 32 columns at once (one
-        // warp per column re-read every row 32 times and was bound by shared-memory bandwidth).
-        constexpr int kSlab = 256, kVp = 36, kPer = kSlab * kPanel / NT;    // row pitch 36: 16-byte aligned rows
-        float pre[kPer];
-        auto fetch = [&](int rb) {
+        const float *Vg = V + (long long)r0 * ld + r0;
+        const int groups = (mu + 31) >> 5;
+        // ---- W = Vp^T C: k runs over the window's rows, 32 at a time; k index tig (tig + 4) of step j is row 8 tig + 2 j (+ 1),
+        // which keeps the shared reads of C conflict-free
+        float av[4][8];
+        auto fetch_v = [&](int gr) {
+            if (gr >= groups) return;
+            const float *vg = Vg + (long long)(32 * gr + 8 * tig) * ld + g;
 #pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-                const int i = tid + q * NT, rr = i >> 5, j = i & 31;
-                pre[q] = (rb + rr < mu && j < prev_w) ? Vg[(long long)(rb + rr) * ld + j] : 0.0f;
-            }
-        };
-        auto stash = [&]() {
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-                const int i = tid + q * NT;
-                Vs[(i >> 5) * kVp + (i & 31)] = pre[q];
-            }
-        };
-        // ---- W = Vp^T C.  Warp (g, h): reflector columns JG g .. JG g + JG - 1, rows h, h+8, .. of each slab.
-        constexpr int JG = kPanel / (NW / 8);
-        const int g8 = (warp >> 3) * JG, h = warp & 7;
-        float wacc[JG];
-#pragma unroll
-        for (int j = 0; j < JG; ++j) wacc[j] = 0.0f;
-        fetch(0);
-        for (int rb = 0; rb < mu; rb += kSlab) {
-            __syncthreads();
-            stash();
-            __syncthreads();
-            fetch(rb + kSlab < mu ? rb + kSlab : 0);       // after the last slab: the first slab of the second pass
-#pragma unroll 4
-            for (int k = 0; k < kSlab / 8; ++k) {
-                const int rr = h + 8 * k;
-                if (rb + rr < mu) {
-                    const float cv = C[(rb + rr) * 33 + lane];
-#pragma unroll
-                    for (int j = 0; j < JG; j += 4) {
-                        const float4 v0 = *reinterpret_cast<const float4 *>(Vs + rr * kVp + g8 + j);
-                        wacc[j] = fmaf(v0.x, cv, wacc[j]); wacc[j + 1] = fmaf(v0.y, cv, wacc[j + 1]);
-                        wacc[j + 2] = fmaf(v0.z, cv, wacc[j + 2]); wacc[j + 3] = fmaf(v0.w, cv, wacc[j + 3]);
-                    }
+                for (int q = 0; q < 8; ++q) {
+                    const int row = 32 * gr + 8 * tig + 2 * j + (q >> 2);
+                    av[j][q] = (row < mu && g + 8 * (q & 3) < prev_w) ? vg[(2 * j + (q >> 2)) * ld + 8 * (q & 3)] : 0.0f;
                 }
+        };
+        fetch_v(warp);
+        __syncthreads();
+        float acc[2][4][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0f;
+        for (int gr = warp; gr < groups; gr += kPw) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                unsigned ah[2][4], al[2][4], bh[4][2], bl[4][2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {              // a0: (g, tig), a1: (g + 8, tig), a2: (g, tig + 4), a3: (g + 8, tig + 4)
+                    tf32_split(av[j][2 * i], ah[i][0], al[i][0]);
+                    tf32_split(av[j][2 * i + 1], ah[i][1], al[i][1]);
+                    tf32_split(av[j][4 + 2 * i], ah[i][2], al[i][2]);
+                    tf32_split(av[j][4 + 2 * i + 1], ah[i][3], al[i][3]);
+                }
+                const float *cr = C + (32 * gr + 8 * tig + 2 * j) * kPp + g;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    tf32_split(cr[8 * t], bh[t][0], bl[t][0]);
+                    tf32_split(cr[kPp + 8 * t], bh[t][1], bl[t][1]);
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) { mma_tf32(acc[0][t], al[0], bh[t]); mma_tf32(acc[1][t], al[1], bh[t]); }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) { mma_tf32(acc[0][t], ah[0], bl[t]); mma_tf32(acc[1][t], ah[1], bl[t]); }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) { mma_tf32(acc[0][t], ah[0], bh[t]); mma_tf32(acc[1][t], ah[1], bh[t]); }
             }
+            fetch_v(gr + kPw);
         }
-        __syncthreads();                                   // the slab buffer is free: it takes the eight partial sums
-        float *Wpart = Vs;                                 // [8 row groups][32][33]
+        // sum of the warps' partial results: eight leave theirs, the other eight add, the eight sums are added by all
+        float *mine = part + (warp & 7) * (32 * 33) + g * 33 + 2 * tig;
 #pragma unroll
-        for (int j = 0; j < JG; ++j) Wpart[(h * kPanel + g8 + j) * 33 + lane] = wacc[j];
-        __syncthreads();
-        float *Wm = G;                                     // [32][33]; G is cleared again before the factorisation
-        for (int jr = warp; jr < kPanel; jr += NW) {
-            float wsum = 0.0f;                             // W[jr][lane]
+        for (int half = 1; half >= 0; --half) {
+            if ((warp >> 3) == half) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) wsum += Wpart[(q * kPanel + jr) * 33 + lane];
-            Wm[jr * 33 + lane] = wsum;
-        }
-        __syncthreads();
-        for (int jr = warp; jr < kPanel; jr += NW) {
-            float z = 0.0f;                                // z[jr][lane] = (Tp^T W)[jr][lane]
+                for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < kPanel; ++j) z = fmaf(Tp[j * (kPanel + 1) + jr], Wm[j * 33 + lane], z);
-            zs[jr * 33 + lane] = z;
-        }
-        __syncthreads();
-        float zreg[kPanel];
+                    for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int j = 0; j < kPanel; ++j) zreg[j] = zs[j * 33 + lane];
-        // ---- C -= Vp z.  Warp w: rows w, w+NW, .. of each slab.
-        for (int rb = 0; rb < mu; rb += kSlab) {
+                        for (int q = 0; q < 4; ++q) {
+                            float *d = mine + (16 * i + 8 * (q >> 1)) * 33 + 8 * t + (q & 1);
+                            if (half) *d = acc[i][t][q]; else *d += acc[i][t][q];
+                        }
+            }
             __syncthreads();
-            stash();
-            __syncthreads();
-            if (rb + kSlab < mu) fetch(rb + kSlab);
-#pragma unroll 2
-            for (int k = 0; k < kSlab / NW; ++k) {
-                const int rr = warp + NW * k;
-                if (rb + rr < mu) {
-                    float a0 = 0.0f, a1 = 0.0f;
+        }
+        for (int jr = warp; jr < 32; jr += kPw) {
+            float s = 0.0f;
 #pragma unroll
-                    for (int j = 0; j < kPanel; j += 8) {
-                        const float4 v0 = *reinterpret_cast<const float4 *>(Vs + rr * kVp + j);
-                        const float4 v1 = *reinterpret_cast<const float4 *>(Vs + rr * kVp + j + 4);
-                        a0 = fmaf(v0.x, zreg[j], a0); a0 = fmaf(v0.y, zreg[j + 1], a0);
-                        a0 = fmaf(v0.z, zreg[j + 2], a0); a0 = fmaf(v0.w, zreg[j + 3], a0);
-                        a1 = fmaf(v1.x, zreg[j + 4], a1); a1 = fmaf(v1.y, zreg[j + 5], a1);
-                        a1 = fmaf(v1.z, zreg[j + 6], a1); a1 = fmaf(v1.w, zreg[j + 7], a1);
+            for (int q = 0; q < 8; ++q) s += part[q * (32 * 33) + jr * 33 + lane];
+            Wm[jr * 33 + lane] = s;
+        }
+        __syncthreads();
+        for (int jr = warp; jr < 32; jr += kPw) {           // z = Tp^T W
+            float z0 = 0.0f, z1 = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+                z0 = fmaf(Tp[j * 33 + jr], Wm[j * 33 + lane], z0);
+                z1 = fmaf(Tp[(j + 1) * 33 + jr], Wm[(j + 1) * 33 + lane], z1);
+            }
+            zs[jr * 33 + lane] = z0 + z1;
+        }
+        __syncthreads();
+        // ---- C -= Vp z, 32 rows at a time: fragment row g (g + 8) of tile rt is row 4 g + 2 rt (+ 1)
+        float zr[4][4][2];                                  // z fragments: k-step, column tile
+#pragma unroll
+        for (int kb = 0; kb < 4; ++kb)
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                zr[kb][t][0] = zs[(8 * kb + tig) * 33 + 8 * t + g];
+                zr[kb][t][1] = zs[(8 * kb + tig + 4) * 33 + 8 * t + g];
+            }
+        for (int gr = warp; gr < groups; gr += kPw) {
+            const int row = 32 * gr + 4 * g;
+            const float *vg = Vg + (long long)row * ld + tig;
+            float up[2][4][4], a[2][4];
+#pragma unroll
+            for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) up[rt][t][q] = 0.0f;
+            auto fetch_a = [&](int kb) {
+#pragma unroll
+                for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int dr = 2 * rt + (q & 1), dc = 8 * kb + 4 * (q >> 1);
+                        a[rt][q] = (row + dr < mu && tig + dc < prev_w) ? vg[dr * ld + dc] : 0.0f;
                     }
-                    C[(rb + rr) * 33 + lane] -= a0 + a1;
+            };
+            fetch_a(0);
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                unsigned ah[2][4], al[2][4], bh[4][2], bl[4][2];
+#pragma unroll
+                for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) tf32_split(a[rt][q], ah[rt][q], al[rt][q]);
+                if (kb < 3) fetch_a(kb + 1);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    tf32_split(zr[kb][t][0], bh[t][0], bl[t][0]);
+                    tf32_split(zr[kb][t][1], bh[t][1], bl[t][1]);
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) { mma_tf32(up[0][t], al[0], bh[t]); mma_tf32(up[1][t], al[1], bh[t]); }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) { mma_tf32(up[0][t], ah[0], bl[t]); mma_tf32(up[1][t], ah[1], bl[t]); }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) { mma_tf32(up[0][t], ah[0], bh[t]); mma_tf32(up[1][t], ah[1], bh[t]); }
+            }
+#pragma unroll
+            for (int rt = 0; rt < 2; ++rt) {
+                float *cr = C + (row + 2 * rt) * kPp + 2 * tig;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    cr[8 * t] -= up[rt][t][0];
+                    cr[8 * t + 1] -= up[rt][t][1];
+                    cr[kPp + 8 * t] -= up[rt][t][2];
+                    cr[kPp + 8 * t + 1] -= up[rt][t][3];
                 }
             }
         }
         __syncthreads();
         if (chunk > 0) {                                   // not the new panel: write the updated chunk back and leave
-            for (int r = warp; r < mu; r += NW)
-                if (lane < wc) Cg[(long long)r * ld + lane] = C[r * 33 + lane];
+#pragma unroll 4
+            for (int r = warp; r < mu; r += kPw)
+                if (lane < wc) Cg[(long long)r * ld + lane] = C[r * kPp + lane];
             return;
         }
-        // chunk 0: rows prev_w.. of the window are the new panel, already in P
-        for (int r = warp; r < m; r += NW)
-            if (lane >= w) P[r * 33 + lane] = 0.0f;
-    } else {
-        for (int r = warp; r < m; r += NW) P[r * 33 + lane] = (lane < w) ? A[(long long)r * ld + lane] : 0.0f;
+        if (w < kPanel)
+            for (int r = warp; r < m; r += kPw)
+                if (lane >= w) P[r * kPp + lane] = 0.0f;
     }
-    for (int i = tid; i < 2 * kPanel * (kPanel + 1); i += NT) G[i] = 0.0f;   // G and Ts are adjacent
+    for (int i = tid; i < 2 * 32 * 33; i += kPt) G[i] = 0.0f;   // G and Ts are adjacent
+    if (tid < 32) tau[tid] = 0.0f;
     __syncthreads();
-    const int cA = 2 * warp, cB = 2 * warp + 1;
+
+    // ---- factorisation
+    const int cA = 2 * warp, cB = cA + 1;
     float colA[RT], colB[RT];
 #pragma unroll
     for (int k = 0; k < RT; ++k) {
-        const int r = lane + 32 * k;
-        colA[k] = (r < m) ? P[r * 33 + cA] : 0.0f;
-        colB[k] = (r < m) ? P[r * 33 + cB] : 0.0f;
+        colA[k] = P[(lane + 32 * k) * kPp + cA];
+        colB[k] = P[(lane + 32 * k) * kPp + cB];
     }
-    float trA = 0.0f, trB = 0.0f;                            // rows cA, cB of T: lane k holds T[row][k]
-    auto t_row = [&](int row, float &tr, int i) {
-        if (row < i) {
-            const float part = (lane >= row && lane < i) ? tr * G[lane * (kPanel + 1) + i] : 0.0f;
-            const float sum = warp_sum(part);
-            if (lane == i) tr = -tau[i] * sum;
-        } else if (row == i && lane == i) {
-            tr = tau[i];
-        }
-    };
-
-    for (int c = 0; c < w; ++c) {
-        float *vbuf = vb + (c & 1) * (RT * 32);
-        const bool odd = (c & 1) != 0;
-        if (warp == (c >> 1)) {
-            float s4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const float *Pl = P + lane * kPp;                      // this lane's rows
+#pragma unroll 1
+    for (int sp = 0; sp < 4 && 8 * sp < w; ++sp) {
+        if ((warp >> 2) == sp) {
+            const int end = min(8 * sp + 8, w);
+            float *xb = part + lane;                          // [2][RT * 32] the pivot column as it is, double-buffered
+            float scA = 0.0f, scB = 0.0f;                     // scalings of this warp's finished pivots
+            if (cA == 8 * sp) {
 #pragma unroll
-            for (int k = 0; k < RT; ++k) {
-                const float x = odd ? colB[k] : colA[k];
-                s4[k & 3] = (lane + 32 * k > c) ? fmaf(x, x, s4[k & 3]) : s4[k & 3];
+                for (int k = 0; k < RT; ++k) xb[32 * k] = colA[k];
             }
-            const float sigma = warp_sum((s4[0] + s4[1]) + (s4[2] + s4[3]));
-            const float alpha = __shfl_sync(0xffffffffu, odd ? colB[0] : colA[0], c);   // row c lives in lane c, slot 0
-            float tc = 0.0f, scale = 0.0f;
-            if (sigma != 0.0f) {
-                const float beta = -copysignf(sqrtf(fmaf(alpha, alpha, sigma)), alpha);
-                tc = (beta - alpha) / beta;
-                scale = 1.0f / (alpha - beta);
-            }
-#pragma unroll
-            for (int k = 0; k < RT; ++k) {
-                const int r = lane + 32 * k;
-                const float x = odd ? colB[k] : colA[k];
-                const float v = (r > c) ? x * scale : (r == c ? 1.0f : 0.0f);
-                if (odd) colB[k] = v; else colA[k] = v;      // the column now holds v_c
-                vbuf[k * 32 + lane] = v;
-            }
-            if (lane == 0) tau[c] = tc;
-        }
-        __syncthreads();
-        if (cA < w) {
-            float a4[2] = {0.0f, 0.0f}, b4[2] = {0.0f, 0.0f};
-#pragma unroll
-            for (int k = 0; k < RT; ++k) {
-                const float vv = vbuf[k * 32 + lane];
-                a4[k & 1] = fmaf(vv, colA[k], a4[k & 1]);
-                b4[k & 1] = fmaf(vv, colB[k], b4[k & 1]);
-            }
-            float dA = a4[0] + a4[1], dB = b4[0] + b4[1];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {         // two reductions interleaved
-                dA += __shfl_xor_sync(0xffffffffu, dA, off);
-                dB += __shfl_xor_sync(0xffffffffu, dB, off);
-            }
-            const float tc = tau[c];
-            const float fA = (cA > c) ? tc * dA : 0.0f;      // columns to the right of c get H_c applied
-            const float fB = (cB > c && cB < w) ? tc * dB : 0.0f;
-            if (cB > c) {                                    // at least column B is updated (warp-uniform)
+#pragma unroll 1
+            for (int c = 8 * sp; c < end; ++c) {
+                const float *xc = xb + (c & 1) * (32 * RT);
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                // one round of reductions: the pivot's norm (every warp for itself) and the products with both columns
+                float s2[2] = {0.0f, 0.0f}, a2[2] = {0.0f, 0.0f}, b2[2] = {0.0f, 0.0f};
 #pragma unroll
                 for (int k = 0; k < RT; ++k) {
-                    const float vv = vbuf[k * 32 + lane];
-                    colA[k] = fmaf(-fA, vv, colA[k]);
-                    colB[k] = fmaf(-fB, vv, colB[k]);
+                    float x = xc[32 * k];
+                    if (k == 0) x = lane > c ? x : 0.0f;
+                    s2[k & 1] = fmaf(x, x, s2[k & 1]);
+                    a2[k & 1] = fmaf(x, colA[k], a2[k & 1]);
+                    b2[k & 1] = fmaf(x, colB[k], b2[k & 1]);
+                }
+                const float alpha = part[(c & 1) * (32 * RT) + c];
+                const float eA = __shfl_sync(0xffffffffu, colA[0], c), eB = __shfl_sync(0xffffffffu, colB[0], c);   // row c: lane c, slot 0
+                float sigma = s2[0] + s2[1], dA = a2[0] + a2[1], dB = b2[0] + b2[1];
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) {
+                    sigma += __shfl_xor_sync(0xffffffffu, sigma, off);
+                    dA += __shfl_xor_sync(0xffffffffu, dA, off);
+                    dB += __shfl_xor_sync(0xffffffffu, dB, off);
+                }
+                // tau = (beta - alpha) / beta, v = (1, scale x): tau * scale = -1 / beta, so the update waits for two
+                // reciprocals side by side and not for a division
+                float rb = 0.0f, scale = 0.0f, diff = 0.0f;
+                if (sigma != 0.0f) {
+                    const float beta = -copysignf(sqrtf(fmaf(alpha, alpha, sigma)), alpha);
+                    diff = beta - alpha;
+                    rb = 1.0f / beta;
+                    scale = -1.0f / diff;
+                }
+                const float tc = diff * rb;
+                dA = fmaf(scale, dA, eA);                     // v . column
+                dB = fmaf(scale, dB, eB);
+                __syncwarp();                                 // x is read again: RT values kept from the products would spill
+                if (cB > c) {                                 // at least column B is updated (warp-uniform)
+                    const float fA = cA > c ? tc * dA : 0.0f, fB = tc * dB;
+                    const float hA = cA > c ? -rb * dA : 0.0f, hB = -rb * dB;
+                    const float x0 = xc[0];
+                    colA[0] = lane > c ? fmaf(-hA, x0, colA[0]) : (lane == c ? colA[0] - fA : colA[0]);
+                    colB[0] = lane > c ? fmaf(-hB, x0, colB[0]) : (lane == c ? colB[0] - fB : colB[0]);
+#pragma unroll
+                    for (int k = 1; k < RT; ++k) {
+                        const float x = xc[32 * k];
+                        colA[k] = fmaf(-hA, x, colA[k]);
+                        colB[k] = fmaf(-hB, x, colB[k]);
+                    }
+                    if (c + 1 < end && warp == ((c + 1) >> 1)) {      // the next pivot
+                        float *xn = xb + ((c + 1) & 1) * (32 * RT);
+#pragma unroll
+                        for (int k = 0; k < RT; ++k) xn[32 * k] = cA == c + 1 ? colA[k] : colB[k];
+                    }
+                }
+                // finished columns are still unscaled: v_col . v_c = scale_col (scale_c x_col . x + x_col[c])
+                if (cA < c && lane == 0) G[cA * 33 + c] = scA * dA;
+                if (cB < c && lane == 0) G[cB * 33 + c] = scB * dB;
+                if (cA == c) scA = scale;
+                if (cB == c) scB = scale;
+                if (warp == (c >> 1) && lane == 0) tau[c] = tc;
+            }
+            if (cA < end) {                                   // the pivots become v
+                float *pub = P + lane * kPp + cA;
+#pragma unroll
+                for (int k = 0; k < RT; ++k) {
+                    colA[k] *= scA;
+                    if (k == 0) colA[0] = lane > cA ? colA[0] : (lane == cA ? 1.0f : 0.0f);
+                    pub[32 * k * kPp] = colA[k];
+                    if (cB < end) {
+                        colB[k] *= scB;
+                        if (k == 0) colB[0] = lane > cB ? colB[0] : (lane == cB ? 1.0f : 0.0f);
+                        pub[32 * k * kPp + 1] = colB[k];
+                    }
                 }
             }
-            if (lane == 0) {                                 // finished columns: v_col . v_c for the triangular factor
-                if (cA < c) G[cA * (kPanel + 1) + c] = dA;
-                if (cB < c) G[cB * (kPanel + 1) + c] = dB;
+        }
+        __syncthreads();                                      // the sub-panel's vectors, tau and products are published
+        // the next sub-panel's warps have shared memory to themselves for their pass; the others follow beside its column steps
+        const bool next = (warp >> 2) == sp + 1;
+        const int s0 = 8 * sp;
+        float z[16];                                          // [column A / B][vector]
+        if (sp < 3 && !next) asm volatile("bar.sync 3, 512;" ::: "memory");
+        if (warp >= 4 * sp + 4 && cA < w) {
+            dot8<RT>(Pl, s0, colA, colB, z, lane);
+            __syncwarp();                                     // the vectors are read again (8 RT values kept would spill)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                float a = z[j], b = z[8 + j];
+#pragma unroll
+                for (int i = 0; i < j; ++i) {
+                    const float gij = G[(s0 + i) * 33 + s0 + j];
+                    a = fmaf(-gij, z[i], a);
+                    b = fmaf(-gij, z[8 + i], b);
+                }
+                const float tj = tau[s0 + j];
+                z[j] = tj * a;
+                z[8 + j] = tj * b;
             }
-            if (c >= 1) { t_row(cA, trA, c - 1); t_row(cB, trB, c - 1); }
+#pragma unroll
+            for (int k = 0; k < RT; ++k)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float v = Pl[32 * k * kPp + s0 + j];
+                    colA[k] = fmaf(-z[j], v, colA[k]);
+                    colB[k] = fmaf(-z[8 + j], v, colB[k]);
+                }
+        } else if (warp < 4 * sp) {                           // finished columns: their products with the new vectors
+            dot8<RT>(Pl, s0, colA, colB, z, lane);
+            if (lane == 0) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) { G[cA * 33 + s0 + j] = z[j]; G[cB * 33 + s0 + j] = z[8 + j]; }
+            }
+        }
+        if (next) asm volatile("bar.arrive 3, 512;" ::: "memory");
+    }
+    __syncthreads();
+    // ---- triangular factor from V^T V and tau (LAPACK slarft): four 8 x 8 blocks, then -T1 (G12 T2) for the off-diagonal
+    // blocks of 8 and of 16.  Eight warps; the others store V meanwhile.  (One warp running down 32 columns took 5600 clocks.)
+    if (warp < 8) {
+        auto sync8 = [] { asm volatile("bar.sync 2, 256;" ::: "memory"); };
+        if (warp < 4 && lane < 8) {
+            const int b = 8 * warp;
+            float t[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float x = 0.0f;
+#pragma unroll
+                for (int k = 0; k < i; ++k) x = fmaf(t[k], G[(b + k) * 33 + b + i], x);   // t[k] is zero for k < lane
+                const float ti = tau[b + i];
+                t[i] = lane < i ? -ti * x : (lane == i ? ti : 0.0f);
+                Ts[(b + lane) * 33 + b + i] = t[i];
+            }
+        }
+        sync8();
+        const int p = 16 * (tid >> 6), pr = p + ((tid >> 3) & 7), pc = p + 8 + (tid & 7);
+        if (tid < 128) {                                      // pairs of 8: Wm = G12 T2
+            float x = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x = fmaf(G[pr * 33 + p + 8 + k], Ts[(p + 8 + k) * 33 + pc], x);
+            Wm[pr * 33 + pc] = x;
+        }
+        sync8();
+        if (tid < 128) {
+            float x = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x = fmaf(Ts[pr * 33 + p + k], Wm[(p + k) * 33 + pc], x);
+            Ts[pr * 33 + pc] = -x;
+        }
+        sync8();
+        const int r = tid >> 4, c = 16 + (tid & 15);          // 256 threads: the 16 x 16 block
+        float x = 0.0f, y = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) x = fmaf(G[r * 33 + 16 + k], Ts[(16 + k) * 33 + c], x);
+        Wm[r * 33 + c] = x;
+        sync8();
+#pragma unroll
+        for (int k = 0; k < 16; ++k) y = fmaf(Ts[r * 33 + k], Wm[k * 33 + c], y);
+        Ts[r * 33 + c] = -y;
+        sync8();
+        float *T = Tbase + (long long)blockIdx.x * strideT;
+        for (int i = tid; i < kPanel * kPanel; i += 256) {
+            const int a = i >> 5, b = i & 31;
+            T[i] = (a < w && b < w) ? Ts[a * 33 + b] : 0.0f;
         }
     }
-    __syncthreads();
-    if (cA < w) { t_row(cA, trA, w - 1); t_row(cB, trB, w - 1); }
-    Ts[cA * (kPanel + 1) + lane] = (lane >= cA && lane < w && cA < w) ? trA : 0.0f;
-    Ts[cB * (kPanel + 1) + lane] = (lane >= cB && lane < w && cB < w) ? trB : 0.0f;
-#pragma unroll
-    for (int k = 0; k < RT; ++k) {
-        const int r = lane + 32 * k;
-        if (r < m) { P[r * 33 + cA] = colA[k]; P[r * 33 + cB] = colB[k]; }
+    float *Vo = V + (long long)j0 * ld + j0;
+#pragma unroll 4
+    for (int r = warp; r < m; r += kPw)
+        if (lane < w) Vo[(long long)r * ld + lane] = P[r * kPp + lane];
+    store_panel_planes(planes, P, m, w, kPw);
+}
+
+template <int RT>
+static int launch_panel(float *A, long long strideA, int n, int ld, int count, int j0, int w, float *V, long long strideV, float *T, long long strideT,
+                        cudaStream_t s, int prev_w, const float *Tprev, int block_end, const PanelPlanes &planes) {
+    const size_t smem = sizeof(float) * ((size_t)(32 * RT + 64) * kPp + 8 * 32 * 33 + 5 * 32 * 33 + 32);
+    static PerDeviceOnce attr_set;
+    const int dev = current_device();
+    if (attr_set.pending(dev)) {
+        if (cudaFuncSetAttribute(k_panel<RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return record(QT_ERR_LAUNCH);
+        attr_set.mark(dev);
     }
-    __syncthreads();
-    float *V = Vbase + (long long)blockIdx.x * strideV + (long long)j0 * ld + j0;
-    for (int r = warp; r < m; r += NW)
-        if (lane < w) V[(long long)r * ld + lane] = P[r * 33 + lane];
-    store_panel_planes(planes, P, m, w, NW);
-    float *T = Tbase + (long long)blockIdx.x * strideT;
-    for (int i = tid; i < kPanel * kPanel; i += NT) T[i] = Ts[(i / kPanel) * (kPanel + 1) + (i % kPanel)];
+    const int chunks = prev_w > 0 ? (block_end - j0 + kPanel - 1) / kPanel : 1;
+    k_panel<RT><<<dim3(count, chunks), kPt, smem, s>>>(A, strideA, n, ld, j0, w, V, strideV, T, strideT, prev_w, Tprev, block_end, planes);
+    count_launch(1);
+    return check_launch();
 }
 
 template <int RPL, int RS>
@@ -593,28 +823,6 @@ static int launch_panel_rpl(float *A, long long strideA, int n, int ld, int coun
     return check_launch();
 }
 
-template <int RT>
-static int launch_panel_pairs(float *A, long long strideA, int n, int ld, int count, int j0, int w,
-                              float *V, long long strideV, float *T, long long strideT, cudaStream_t s,
-                              int prev_w, const float *Tprev, int block_end, const PanelPlanes &planes) {
-    const int m = n - j0;
-    const size_t smem = sizeof(float) * ((size_t)(((kPanel + m) * 33 + 31) & ~31) + 2 * RT * 32 + 2 * kPanel * (kPanel + 1) + kPanel +
-                                         256 * 36 + kPanel * (kPanel + 1) + kPanel * (kPanel + 1));
-    static PerDeviceOnce attr_set;
-    const int dev = current_device();
-    if (attr_set.pending(dev)) {
-        if (cudaFuncSetAttribute(k_householder_panel_pairs<RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
-            return record(QT_ERR_LAUNCH);
-        attr_set.mark(dev);
-    }
-    if (smem > 227 * 1024) return record(QT_ERR_UNSUPPORTED);
-    const int chunks = prev_w > 0 ? (block_end - j0 + kPanel - 1) / kPanel : 1;
-    dim3 grid(count, chunks);
-    k_householder_panel_pairs<RT><<<grid, 512, smem, s>>>(A, strideA, n, ld, j0, w, V, strideV, T, strideT, prev_w, Tprev, block_end, planes);
-    count_launch(1);
-    return check_launch();
-}
-
 int launch_householder_panel(float *A, long long strideA, int n, int ld, int count, int j0, int w,
                              float *V, long long strideV, float *T, long long strideT, cudaStream_t s,
                              int prev_w, const float *Tprev, int block_end,
@@ -629,17 +837,22 @@ int launch_householder_panel(float *A, long long strideA, int n, int ld, int cou
     if (count > 65535) return record(QT_ERR_UNSUPPORTED);
     const int rows_per_lane = (n - j0 + 31) / 32;
     if (rows_per_lane > kMaxRowsPerLane) return record(QT_ERR_UNSUPPORTED);
-#define QT_PANEL(R, S) return launch_panel_rpl<R, S>(A, strideA, n, ld, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end, planes)
-    if (rows_per_lane <= 6) QT_PANEL(6, 0);
-    if (rows_per_lane <= 12) QT_PANEL(12, 0);
-    if (rows_per_lane <= 20) QT_PANEL(20, 0);
-    if (g_panel_pairs && rows_per_lane > 20) {
-        if (rows_per_lane <= 28) return launch_panel_pairs<28>(A, strideA, n, ld, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end, planes);
-        return launch_panel_pairs<38>(A, strideA, n, ld, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end, planes);
+#define QT_ARGS A, strideA, n, ld, count, j0, w, V, strideV, T, strideT, s, prev_w, Tprev, block_end, planes
+    if (!g_panel_blocked) {
+        if (rows_per_lane <= 20) return launch_panel_rpl<20, 0>(QT_ARGS);
+        return launch_panel_rpl<24, 14>(QT_ARGS);
     }
-    if (rows_per_lane <= 28) QT_PANEL(24, 4);
-    QT_PANEL(24, 14);
-#undef QT_PANEL
+    // rows per lane are rounded up to a multiple of four: the factorisation's time goes with them
+    if (rows_per_lane <= 4) return launch_panel<4>(QT_ARGS);
+    if (rows_per_lane <= 8) return launch_panel<8>(QT_ARGS);
+    if (rows_per_lane <= 12) return launch_panel<12>(QT_ARGS);
+    if (rows_per_lane <= 16) return launch_panel<16>(QT_ARGS);
+    if (rows_per_lane <= 20) return launch_panel<20>(QT_ARGS);
+    if (rows_per_lane <= 24) return launch_panel<24>(QT_ARGS);
+    if (rows_per_lane <= 28) return launch_panel<28>(QT_ARGS);
+    if (rows_per_lane <= 32) return launch_panel<32>(QT_ARGS);
+    return launch_panel<38>(QT_ARGS);
+#undef QT_ARGS
 }
 
 // Triangular factor of an outer block of up to four panels from the panels' own factors and

@@ -94,6 +94,19 @@ def test_both_tall_panel_kernels_agree(native_lib, n):
     check(X)
 
 
+@pytest.mark.parametrize("n", [33, 65, 129, 257, 391, 520, 641, 777, 897, 1025, 1216])
+def test_panel_kernel_at_the_edges_of_its_row_classes(native_lib, n):
+    """One instantiation per 128 rows and the largest order; last panels of 1 to 32 columns, orders
+    with and without vector access.  A zero column keeps its reflector at the identity."""
+    g = torch.Generator(device="cuda").manual_seed(5 * n)
+    X = torch.randn(2, n, n, device="cuda", generator=g)
+    Q, Qt = check(X)
+    rel = float(((Q - Qt).flatten(1).norm(dim=1) / Qt.flatten(1).norm(dim=1)).max())
+    assert rel < TOL, rel
+    X[1, :, n // 2] = 0.0
+    check(X)
+
+
 def test_orders_beyond_the_panel_kernel_fall_back_with_a_warning(native_lib):
     """A panel of more than 1216 rows does not fit one SM's shared memory: such orders go to
     torch.linalg.qr, and say so once."""
