@@ -1440,9 +1440,8 @@ int launch_newton_product(void *const A[3], const int *a_slot, int a_entries,
     x.Thi = T[0]; x.Tmid = T[1]; x.Tlo = T[2]; x.t_c0 = t_c0; x.t_c1 = t_c1;
     x.maxdev = maxdev; x.a_slot = a_slot; x.b_slot = b_slot; x.d_slot = d_slot; x.active = active;
     x.a_entries = a_entries; x.b_entries = b_entries;
-    // every iterate is a polynomial of one symmetric matrix: half of the tiles, mirrored (the asymmetry that full products
-    // accumulate is rounding).  6 x 1200^3 and 6 x 768^3: 110 -> 66 us per product.
-    x.sym = 1;
+    // All tiles: a statistic that comes back from row-blocked 4-bit state differs from its transpose by quantization noise,
+    // and so do the iterates, so mirrored halves would be other results.
     return launch_gemm_planes(a, A[1], B[1], s, nullptr, &x);
 }
 

@@ -338,11 +338,10 @@ def op_ema_gram_selected(L, sel, G, axis, w1, w2):
     operand and writes its result through the slot list, so the selected matrices are neither
     gathered into a temporary nor scattered back (sel: int32 device tensor).  Where products have to be
     exact (_EXACT) the operands are three bf16 planes, 24 bits, instead of an fp32 library product on the
-    SIMT units; the Gram matrix is symmetric, so half of its tiles are computed (6 + 6 matrices of 1200 and 768:
-    430 us of library products, 100 of gathers -> 90 us)."""
+    SIMT units.  All tiles are computed: L comes from row-blocked 4-bit state and is not quite symmetric."""
     P = Mat(G).planes if _tc(L) else Mat(G).planes3
     _gemm.gemm_ex(P, P, trans_a=(axis == 1), trans_b=(axis == 0), alpha=w2, beta=w1, C=L, D=L,
-                  d_slot=sel, c_follows_d=True, batch=G.shape[0], sym=True)
+                  d_slot=sel, c_follows_d=True, batch=G.shape[0])
     return L
 
 
