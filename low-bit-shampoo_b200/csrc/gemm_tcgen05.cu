@@ -57,7 +57,14 @@ template <int NP, int BN_, int EC, bool CONV = false, bool PAIR = false> struct 
     static constexpr int EPI_WARPS = 4 * (BN_ / EC);
     // CONV: four more warps that build an operand's tiles in shared memory from 4-bit state
     static constexpr int CONV_WARPS = CONV ? 4 : 0;
-    static constexpr int THREADS = (EPI_WARPS + 2 + CONV_WARPS) * 32;
+    // Two idle warps complete the producers' warpgroup where there are no converters, so that registers can be moved from
+    // it to the epilogue's two warpgroups (REGS): ten warps get 168 each whatever their role, and partial sums of 96
+    // columns (or 64 and two groups of C in flight) spilled 130 to 320 bytes a thread inside every chain's addition.
+    // 124 x 768^3, D only / D and planes: 337 / 521 -> 321 / 416 us; 62 x 1200^3 with C, D and planes 982 -> 872.
+    static constexpr bool REGS = !CONV && EPI_WARPS == 8;
+    static constexpr int THREADS = (EPI_WARPS + (REGS ? 4 : 2) + CONV_WARPS) * 32;
+    // launch: 384 x 168 = 64512 registers = 256 x EPI_REGS + 128 x PRODUCER_REGS
+    static constexpr int EPI_REGS = 224, PRODUCER_REGS = 56;
     // The whole tensor memory of the SM (one CTA per SM) as a ring of accumulators: four of 128
     // columns, two of 256.  With accumulation chains of 128 k an accumulator is busy for 0.8 us of
     // MMAs only, and the epilogue warps are away for microseconds while they store a finished tile;
@@ -414,7 +421,8 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // a wait that expired in an earlier CTA (or launch) poisons the rest of the grid: drain fast
     // (not in a pair: the two CTAs could decide differently, and one would wait for the other)
-    if (!PAIR && *reinterpret_cast<volatile int *>(&g_gemm_error) != 0) return;
+    // all threads or none: the epilogue's warps wait for the registers that the other warpgroup hands over
+    if (__syncthreads_or(!PAIR && *reinterpret_cast<volatile int *>(&g_gemm_error) != 0)) return;
     const int num_kb = (p.K + BK - 1) / BK;
     const int num_tiles = (p.sym ? p.tiles_m * (p.tiles_m + 1) / 2 : p.tiles_m * p.tiles_n) * p.batch;
     const int nchunks = (num_kb + KC - 1) / KC;
@@ -458,6 +466,9 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
     // does not change while the kernel runs), so their ring and accumulator counters stay in step.
     auto skipped = [&](int b) { return p.active != nullptr && __ldg(p.active + b) == 0; };
 
+    // each branch starts with its register count: behind a common join the compiler keeps to the smaller one
+    if (warp >= EPI_WARPS) {
+    if constexpr (Cfg::REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::PRODUCER_REGS));
     if (warp == EPI_WARPS) {
         // ---------------- TMA producer: one ring of stages shared by all tiles of this CTA
         if (lane == 0) {
@@ -599,7 +610,52 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
                 }
             }
         }
-    } else if (warp < EPI_WARPS) {
+    } else if (CONV && (conv_a || conv_b)) {
+        // ---------------- converter warps: the operand that lives as 4-bit state is dequantized
+        // here, straight into the swizzled tile the tensor core reads - the state's fp32 form and
+        // its operand planes never exist in device memory.  Thread t builds one 128-byte line:
+        // A (row-major, K contiguous): tile row t, the quantization block at columns k0 .. k0+63;
+        // B (row-major, N contiguous): k-row t & 63 of the 64-column chunk t >> 6.
+        const int t = threadIdx.x - (EPI_WARPS + 2) * 32;
+        unsigned it = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+            int tm, tn, b;
+            tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn, b);
+            if (skipped(b)) continue;
+            const int m0 = tm * BM, n0 = tn * BN_;
+            const int sa = conv_a ? (p.aq.slots ? __ldg(p.aq.slots + b) : b) : 0;
+            const int sb = conv_b ? (p.bq.slots ? __ldg(p.bq.slots + b) : b) : 0;
+            const float ea = conv_a ? exp2f((float)(p.a_exp ? __ldg(p.a_exp + b) : 0)) : 1.0f;
+            const float eb = conv_b ? exp2f((float)(p.b_exp ? __ldg(p.b_exp + b) : 0)) : 1.0f;
+            for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                const int s = it % STAGES;
+                ok = mbar_wait_warp(empty_bar(s), ((it / STAGES) & 1) ^ 1, abort_flag);
+                if (!ok) break;
+                const unsigned stage = base + s * STAGE_BYTES;
+                const int k0 = kb * BK;
+                if (conv_a) {
+                    const int row = m0 + t;
+                    const int nvalid = row < p.M ? max(0, min(64, p.K - k0)) : 0;
+                    const unsigned line = stage + (unsigned)t * 128u;
+                    convert_q4_row(p.aq, conv_code, sa, row, k0, nvalid, ea, line, line + PLANE_TILE_BYTES, t);
+                }
+                if (conv_b) {
+                    const int kr = t & 63, chunk = t >> 6;
+                    const int krow = k0 + kr, col = n0 + 64 * chunk;
+                    const int nvalid = krow < p.K ? max(0, min(64, p.N - col)) : 0;
+                    const unsigned line = stage + NP * PLANE_TILE_BYTES + (unsigned)chunk * (PLANE_TILE_BYTES / 2) + (unsigned)kr * 128u;
+                    convert_q4_row(p.bq, conv_code, sb, krow, col, nvalid, eb, line, line + B_PLANE_BYTES, kr);
+                }
+                // make the generic-proxy writes visible to the tensor core's (async-proxy) reads
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full_bar(s)) : "memory");
+            }
+        }
+    }
+    } else {
+        if constexpr (Cfg::REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::EPI_REGS));
         // ---------------- epilogue: warp e reads TMEM lanes 32 (e & 3) .. +31 (lane = output row) and
         // the 128 accumulator columns [128 (e >> 2), +128) of the tile.  Partial sums of the chunks
         // are added in registers; the final combine / conversion / store works on 16 columns at a
@@ -807,49 +863,6 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    } else if (CONV && (conv_a || conv_b)) {
-        // ---------------- converter warps: the operand that lives as 4-bit state is dequantized
-        // here, straight into the swizzled tile the tensor core reads - the state's fp32 form and
-        // its operand planes never exist in device memory.  Thread t builds one 128-byte line:
-        // A (row-major, K contiguous): tile row t, the quantization block at columns k0 .. k0+63;
-        // B (row-major, N contiguous): k-row t & 63 of the 64-column chunk t >> 6.
-        const int t = threadIdx.x - (EPI_WARPS + 2) * 32;
-        unsigned it = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-            int tm, tn, b;
-            tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn, b);
-            if (skipped(b)) continue;
-            const int m0 = tm * BM, n0 = tn * BN_;
-            const int sa = conv_a ? (p.aq.slots ? __ldg(p.aq.slots + b) : b) : 0;
-            const int sb = conv_b ? (p.bq.slots ? __ldg(p.bq.slots + b) : b) : 0;
-            const float ea = conv_a ? exp2f((float)(p.a_exp ? __ldg(p.a_exp + b) : 0)) : 1.0f;
-            const float eb = conv_b ? exp2f((float)(p.b_exp ? __ldg(p.b_exp + b) : 0)) : 1.0f;
-            for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                const int s = it % STAGES;
-                ok = mbar_wait_warp(empty_bar(s), ((it / STAGES) & 1) ^ 1, abort_flag);
-                if (!ok) break;
-                const unsigned stage = base + s * STAGE_BYTES;
-                const int k0 = kb * BK;
-                if (conv_a) {
-                    const int row = m0 + t;
-                    const int nvalid = row < p.M ? max(0, min(64, p.K - k0)) : 0;
-                    const unsigned line = stage + (unsigned)t * 128u;
-                    convert_q4_row(p.aq, conv_code, sa, row, k0, nvalid, ea, line, line + PLANE_TILE_BYTES, t);
-                }
-                if (conv_b) {
-                    const int kr = t & 63, chunk = t >> 6;
-                    const int krow = k0 + kr, col = n0 + 64 * chunk;
-                    const int nvalid = krow < p.K ? max(0, min(64, p.N - col)) : 0;
-                    const unsigned line = stage + NP * PLANE_TILE_BYTES + (unsigned)chunk * (PLANE_TILE_BYTES / 2) + (unsigned)kr * 128u;
-                    convert_q4_row(p.bq, conv_code, sb, krow, col, nvalid, eb, line, line + B_PLANE_BYTES, kr);
-                }
-                // make the generic-proxy writes visible to the tensor core's (async-proxy) reads
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full_bar(s)) : "memory");
-            }
-        }
     }
     __syncthreads();
     if constexpr (PAIR) cluster_sync_all();                   // neither CTA frees or leaves while its peer still works
