@@ -1348,24 +1348,31 @@ int launch_gemm_planes(const GemmArgs &a, const void *Amid, const void *Bmid, cu
     if (!prepare_kernels()) return record(QT_ERR_LAUNCH);
     const int sms = device_sm_count();
     const int tiles_m = (a.M + BM - 1) / BM;
-    // Tile configuration.  The narrow tile with eight epilogue warps is the default: it holds a
-    // thread's 64 partial sums without spilling and keeps twice the loads in flight for epilogues that
-    // stream C, D and planes.  The wide tile needs 25 % less operand traffic per flop (the 128 x 128
-    // tile is bound by operand delivery from L2) and is faster on a plain long-K product (280 vs
-    // 289 us on 125 x 768^3), but its epilogue threads hold 128 partial sums and spill at the 168
-    // registers a 320-thread CTA leaves them; over the whole optimizer step it loses 0.6 ms.  It
-    // stays selectable (qt_gemm_force_tile) for measurements.
+    // Tile width.  What a tile costs is linear in K: per k the time to deliver its operands from L2 (the bound of all three
+    // widths: 25 and 37 % less traffic per result with 192 and 256 columns than with 128), and a share of its epilogue
+    // that the next tile's products do not hide - small for 128 columns, whose four accumulators let the products run
+    // ahead, large for 192 and 256, which have two.  Whole rounds of tiles over the SMs decide, so a few matrices often
+    // do better on narrow tiles.  Microseconds measured on 124 x 768^3 / 124 x (768 x 768 x 384):
+    //   fp32 result only          128: 379 / 204   192: 322 / 181   256: 324 / 190   (62 x 1200^3: 863, 729, 647)
+    //   planes only, or C and D   128: 382 / 216   192: 405 / 263   256: 466 / 293   (62 x 1200^3: 860, 820, 798)
+    //   more streams than that    128: 399 / 253   192: 471 / 301   256: 638 / 401   (C, D, planes: 475, 666, 756)
     int cfg = np == 3 ? 2 : 0;
-    if (np == 2 && a.N > 128 && g_force_bn == 256 && !x.sym && !x.cd_part) cfg = 1;
-    // 128 x 192 tiles (eight epilogue warps of 96 columns, two operand stages, two accumulators): 17 % less
-    // operand traffic per flop than 128 x 128 and, unlike 128 x 256, the 96 partial sums per thread
-    // (nearly) fit the register budget.  Measured against 128 x 128: 125 x 768^3 371 -> 332 us,
-    // 62 x 1200^3 868 -> 748, 36 x (768 x 3072 x 768) 489 -> 402, 8 x 4096^3 3653 -> 2882; with two
-    // k-blocks only (1200 x 1200 x 128) it loses (169 -> 180), so short products stay on 128 x 128.
-    // Products whose epilogue reads C and writes both fp32 and planes stay on 128 x 128 as well (the wide
-    // epilogue is out of registers there: 600 x 1200 x 600 with all three 1.01 -> 1.10 ms per four launches).
-    const bool heavy_epilogue = a.C && a.beta != 0.0f && a.D && a.Dhi;
-    if (np == 2 && a.N > 128 && !qs && !x.sym && (g_force_bn == 192 || (g_force_bn == -1 && a.K >= 256 && !heavy_epilogue))) cfg = 5;
+    if (np == 2 && a.N > 128 && !x.sym) {
+        const int streams = (a.C && a.beta != 0.0f && !x.cd_part ? 1 : 0) + (a.D ? 1 : 0) + (a.Dhi ? 2 : 0);
+        if (g_force_bn >= 0) {
+            if (g_force_bn == 256 && !x.cd_part) cfg = 1;
+            if (g_force_bn == 192 && !qs) cfg = 5;
+        } else if (!qs && streams <= 2) {
+            const int slots = x.max_ctas > 0 && x.max_ctas < sms ? x.max_ctas : sms;
+            auto cost = [&](int width, float per_k, float light, float loaded) {
+                const long long tiles = (long long)tiles_m * ((a.N + width - 1) / width) * a.batch;
+                return (float)((tiles + slots - 1) / slots) * (per_k * (float)a.K + (streams <= 1 ? light : loaded));
+            };
+            const float c128 = cost(128, 0.0147f, 1.0f, 2.0f), c192 = cost(192, 0.0174f, 1.9f, 6.6f), c256 = cost(256, 0.0215f, 3.5f, 11.0f);
+            if (c192 < c128) cfg = 5;
+            if (!x.cd_part && c256 < c128 && c256 < c192) cfg = 1;
+        }
+    }
     if (qa || qb) cfg = 3;
     // CTA pairs (256-row bands) only on request: measured on B200 they are no faster than single
     // CTAs on 128 x 128 tiles (125 x 768^3: 372 vs 364 us; 8 x 4096^3: 3980 vs 3480 us) - halving

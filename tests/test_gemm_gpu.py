@@ -366,3 +366,29 @@ def test_symmetric_product_equals_the_full_product(native_lib, n, k, planes):
     for x, y in zip(out[True], out[False]):
         assert float((x - y).abs().max()) <= 3e-6 * float(y.abs().max())
     assert torch.equal(out[True][0][[1, 3]], C0[[1, 3]])
+
+
+@pytest.mark.parametrize("tile", [192, 256])
+@pytest.mark.parametrize("b,m,n,k", [(2, 130, 136, 72), (1, 128, 193, 256), (3, 257, 449, 200), (2, 300, 520, 1200)])
+def test_wide_tiles_give_the_same_bits(native_lib, tile, b, m, n, k):
+    """The tile width is chosen by size: an element's products and their order do not depend on it."""
+    from optimizers import _gemm
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    A = _gemm.split(torch.randn(b, m, k, device="cuda", generator=g))
+    B = _gemm.split(torch.randn(b, k, n, device="cuda", generator=g))
+    C = torch.randn(b, m, n, device="cuda", generator=g)
+    out = {}
+    for width in (128, tile):
+        native_lib.qt_gemm_force_tile(width)
+        try:
+            D, E = torch.empty_like(C), torch.empty_like(C)
+            P = _gemm.Planes(b, m, n, "cuda", planes=2, f16=True)
+            P.exp0 = 2
+            _gemm.gemm_ex(A, B, D=D)
+            _gemm.gemm_ex(A, B, alpha=0.5, beta=2.0, C=C, D=E)
+            _gemm.gemm_ex(A, B, P=P, out_exp0=2)
+            out[width] = D, E, P.to_float()
+        finally:
+            native_lib.qt_gemm_force_tile(-1)
+    for x, y in zip(out[128], out[tile]):
+        assert torch.equal(x, y)
