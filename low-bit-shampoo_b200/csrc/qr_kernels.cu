@@ -856,85 +856,140 @@ int launch_householder_panel(float *A, long long strideA, int n, int ld, int cou
 }
 
 // Triangular factor of an outer block of up to four panels from the panels' own factors and
-// the Gram matrix G = Vo^T Vo of the block's Householder vectors (LAPACK larft recurrence on
-// blocks): with c columns done and the next panel k of width w,
-//     T[:c, c:c+w] = -T[:c, :c] * G[:c, c:c+w] * T_k,   T[c:c+w, c:c+w] = T_k.
-// One CTA per matrix; T (<= 128 x 128) is assembled in shared memory and written out whole
-// (zeros below the diagonal blocks).  Replaces ~17 small library launches per outer block.
-static constexpr int kMergeMax = 128;
+// the Gram matrix G = Vo^T Vo of the block's Householder vectors (LAPACK larft on blocks, by halves):
+//     T = [T1, -T1 (G12 T2); 0, T2],   first for the two pairs of 32 columns, then for the pair of 64.
+// One CTA per matrix; everything is padded with zeros to 128 columns in shared memory and T is written out whole (zeros
+// below the diagonal blocks).  Bound by latency and by shared-memory wavefronts: the chain is two products of 32^3 and two of
+// 64^3 where panel after panel took three pairs of products that grew with the columns done, and a warp's tile of 8 rows
+// x 16 columns reads four k of a row and of four columns at a time, conflict-free: 5 wavefronts per 4 x 128
+// multiply-adds (one operand and one wavefront per multiply-add before).  27 -> 12 us.
+static constexpr int kMergeMax = 128, kMergeP = 132;         // row pitch: 16-byte rows, 8 rows meet 32 banks
+
+// out[i][j] (+)= sgn * sum over l in [l0, l1) of A[i][l] B[l][j], for this lane's row i and columns j .. j+3
+__device__ __forceinline__ float4 merge_dot(const float *a, const float *b, int l0, int l1) {
+    float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int l = l0; l < l1; l += 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(a + l);
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 y = *reinterpret_cast<const float4 *>(b + (l + q) * kMergeP);
+            r.x = fmaf(xs[q], y.x, r.x); r.y = fmaf(xs[q], y.y, r.y);
+            r.z = fmaf(xs[q], y.z, r.z); r.w = fmaf(xs[q], y.w, r.w);
+        }
+    }
+    return r;
+}
+
 __global__ void __launch_bounds__(1024)
 k_merge_t(const float *__restrict__ Gbase, long long ldg, long long strideG,
           const float *__restrict__ Tp_base, long long strideTp, int wo,
           float *__restrict__ Tbase, long long strideT,
           __half *__restrict__ hi, __half *__restrict__ lo, long long ldp, long long strideP, int *__restrict__ exp_out, int target) {
-    extern __shared__ float merge_sm[];
-    float (*Ts)[kMergeMax + 1] = reinterpret_cast<float (*)[kMergeMax + 1]>(merge_sm);
-    float (*M1)[kPanel + 1] = reinterpret_cast<float (*)[kPanel + 1]>(merge_sm + kMergeMax * (kMergeMax + 1));
-    float (*Tk)[kPanel + 1] = reinterpret_cast<float (*)[kPanel + 1]>(merge_sm + kMergeMax * (kMergeMax + 1) + 96 * (kPanel + 1));
-    // the Gram matrix is staged once: the recurrence below reads each entry in a dependent chain
-    float (*Gs)[kMergeMax + 1] = reinterpret_cast<float (*)[kMergeMax + 1]>(merge_sm + kMergeMax * (kMergeMax + 1) + 96 * (kPanel + 1) +
-                                                                            kPanel * (kPanel + 1));
+    extern __shared__ __align__(16) float merge_sm[];
+    float *Ts = merge_sm, *Gs = Ts + kMergeMax * kMergeP, *red = Gs + kMergeMax * kMergeP;
     const float *G = Gbase + (long long)blockIdx.x * strideG;
     const float *Tp = Tp_base + (long long)blockIdx.x * strideTp;
-    float *T = Tbase + (long long)blockIdx.x * strideT;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;      // warp ty works on rows ty, ty+32, ..; lane = column
-    for (int i = ty; i < wo; i += 32)
-        for (int j = tx; j < wo; j += 32) { Ts[i][j] = 0.0f; Gs[i][j] = __ldg(G + (long long)i * ldg + j); }
-    __syncthreads();
-    for (int c = 0, k = 0; c < wo; c += kPanel, ++k) {
-        const int w = min(kPanel, wo - c);
-        Tk[ty][tx] = (ty < w && tx < w) ? Tp[(long long)k * kPanel * kPanel + ty * kPanel + tx] : 0.0f;
-        __syncthreads();
-        if (ty < w && tx < w) Ts[c + ty][c + tx] = Tk[ty][tx];
-        if (c > 0) {
-            for (int i = ty; i < c; i += 32) {                   // M1 = T[:c, :c] G[:c, c:c+w]; T is upper triangular
-                float acc = 0.0f, acc1 = 0.0f;
-                if (tx < w) {
-                    int l = i;
-                    for (; l + 1 < c; l += 2) {
-                        acc = fmaf(Ts[i][l], Gs[l][c + tx], acc);
-                        acc1 = fmaf(Ts[i][l + 1], Gs[l + 1][c + tx], acc1);
-                    }
-                    if (l < c) acc = fmaf(Ts[i][l], Gs[l][c + tx], acc);
-                }
-                M1[i][tx] = acc + acc1;
-            }
-            __syncthreads();
-            for (int i = ty; i < c; i += 32) {                   // T[:c, c:c+w] = -M1 T_k; T_k is upper triangular
-                float acc = 0.0f;
-                for (int l = 0; l <= tx; ++l) acc = fmaf(M1[i][l], Tk[l][tx], acc);
-                if (tx < w) Ts[i][c + tx] = -acc;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // the panels' factors on the diagonal, zeros elsewhere; the Gram matrix's blocks above the diagonal
+    const bool vec_g = (ldg & 3) == 0 && (strideG & 3) == 0 && (reinterpret_cast<uintptr_t>(Gbase) & 15) == 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int e = tid + 1024 * u, i = e >> 5, j = (e & 31) * 4;
+        float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f), g = t;
+        float ts[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if ((i >> 5) == (j >> 5) && i < wo) {
+            const float *src = Tp + (long long)(i >> 5) * kPanel * kPanel + (i & 31) * kPanel + (j & 31);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) if (j + q < wo) ts[q] = src[q];
+        }
+        if ((j >> 5) > (i >> 5) && i < wo) {
+            const float *src = G + (long long)i * ldg + j;
+            if (vec_g && j + 3 < wo) { g = __ldg(reinterpret_cast<const float4 *>(src)); gs[0] = g.x; gs[1] = g.y; gs[2] = g.z; gs[3] = g.w; }
+            else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) if (j + q < wo) gs[q] = __ldg(src + q);
             }
         }
+        t = make_float4(ts[0], ts[1], ts[2], ts[3]);
+        g = make_float4(gs[0], gs[1], gs[2], gs[3]);
+        *reinterpret_cast<float4 *>(Ts + i * kMergeP + j) = t;
+        *reinterpret_cast<float4 *>(Gs + i * kMergeP + j) = g;
+    }
+    __syncthreads();
+    // pairs of 32 columns at b = 0 and 64: eight warps each; the intermediate product lies below G's diagonal
+    const int b = 64 * (warp >> 3), w8 = warp & 7;
+    const int i1 = 8 * (w8 & 3) + (lane >> 2), j1 = 16 * (w8 >> 2) + 4 * (lane & 3);
+    const bool one = warp < 16 && b + 32 < wo;
+    if (one) *reinterpret_cast<float4 *>(Gs + (b + 32 + i1) * kMergeP + b + j1) =
+                 merge_dot(Gs + (b + i1) * kMergeP + b + 32, Ts + (b + 32) * kMergeP + b + 32 + j1, 0, 16 * (w8 >> 2) + 16);   // T2 is upper triangular
+    __syncthreads();
+    if (one) {
+        const float4 r = merge_dot(Ts + (b + i1) * kMergeP + b, Gs + (b + 32) * kMergeP + b + j1, 8 * (w8 & 3), 32);           // and T1
+        *reinterpret_cast<float4 *>(Ts + (b + i1) * kMergeP + b + 32 + j1) = make_float4(-r.x, -r.y, -r.z, -r.w);
+    }
+    __syncthreads();
+    if (wo > 64) {                                            // the pair of 64: all warps
+        const int i2 = 8 * (warp & 7) + (lane >> 2), j2 = 16 * (warp >> 3) + 4 * (lane & 3);
+        *reinterpret_cast<float4 *>(Gs + (64 + i2) * kMergeP + j2) = merge_dot(Gs + i2 * kMergeP + 64, Ts + 64 * kMergeP + 64 + j2, 0, 16 * (warp >> 3) + 16);
+        __syncthreads();
+        const float4 r = merge_dot(Ts + i2 * kMergeP, Gs + 64 * kMergeP + j2, 8 * (warp & 7), 64);
+        *reinterpret_cast<float4 *>(Ts + i2 * kMergeP + 64 + j2) = make_float4(-r.x, -r.y, -r.z, -r.w);
         __syncthreads();
     }
-    if (Tbase)
-        for (int i = ty; i < wo; i += 32)
-            for (int j = tx; j < wo; j += 32) T[(long long)i * wo + j] = Ts[i][j];
+    if (Tbase) {
+        float *T = Tbase + (long long)blockIdx.x * strideT;
+        for (int i = warp; i < wo; i += 32)
+            for (int j = lane; j < wo; j += 32) T[(long long)i * wo + j] = Ts[i * kMergeP + j];
+    }
     if (!hi) return;
     // scaled fp16 planes of T (the operand of the products that follow), exponent from the largest magnitude
-    float am = 0.0f;
-    for (int i = ty; i < wo; i += 32)
-        for (int j = tx; j < wo; j += 32) am = fmaxf(am, fabsf(Ts[i][j]));
+    float v[2][8], am = 0.0f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int e = tid + 1024 * u, i = e >> 4, j = (e & 15) * 8;
+#pragma unroll
+        for (int q = 0; q < 8; q += 4) {
+            const float4 x = *reinterpret_cast<const float4 *>(Ts + i * kMergeP + j + q);
+            v[u][q] = x.x; v[u][q + 1] = x.y; v[u][q + 2] = x.z; v[u][q + 3] = x.w;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) am = fmaxf(am, fabsf(v[u][q]));
+    }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, off));
-    if (tx == 0) M1[0][ty] = am;
+    if (lane == 0) red[warp] = am;
     __syncthreads();
-    am = M1[0][tx];
+    am = red[lane];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, off));
-    const int e = exponent_for(am, target);
-    if (threadIdx.x == 0) exp_out[blockIdx.x] = e;
-    const float two_e = exp2f((float)e);
+    const int e_out = exponent_for(am, target);
+    if (tid == 0) exp_out[blockIdx.x] = e_out;
+    const float two_e = exp2f((float)e_out);
     hi += (long long)blockIdx.x * strideP;
     lo += (long long)blockIdx.x * strideP;
-    for (int i = ty; i < wo; i += 32)
-        for (int j = tx; j < wo; j += 32) {
-            const float x = fminf(fmaxf(Ts[i][j] * two_e, -65000.0f), 65000.0f);
-            const __half h = __float2half_rn(x);
-            hi[(long long)i * ldp + j] = h;
-            lo[(long long)i * ldp + j] = __float2half_rn(x - __half2float(h));
+    const bool vec_p = ((ldp | strideP) & 7) == 0 && ((reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15) == 0;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int e = tid + 1024 * u, i = e >> 4, j = (e & 15) * 8;
+        if (i >= wo || j >= wo) continue;
+        __half h[8], l[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float x = fminf(fmaxf(v[u][q] * two_e, -65000.0f), 65000.0f);
+            h[q] = __float2half_rn(x);
+            l[q] = __float2half_rn(x - __half2float(h[q]));
         }
+        __half *dh = hi + (long long)i * ldp + j, *dl = lo + (long long)i * ldp + j;
+        if (vec_p && j + 8 <= wo) {
+            auto word = [](const __half *p) { return (unsigned)__half_as_ushort(p[0]) | ((unsigned)__half_as_ushort(p[1]) << 16); };
+            *reinterpret_cast<uint4 *>(dh) = make_uint4(word(h), word(h + 2), word(h + 4), word(h + 6));
+            *reinterpret_cast<uint4 *>(dl) = make_uint4(word(l), word(l + 2), word(l + 4), word(l + 6));
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) if (j + q < wo) { dh[q] = h[q]; dl[q] = l[q]; }
+        }
+    }
 }
 
 int launch_merge_t(const float *G, long long ldg, long long strideG, const float *Tp, long long strideTp, int wo, int count,
@@ -942,7 +997,7 @@ int launch_merge_t(const float *G, long long ldg, long long strideG, const float
     if (wo <= 0 || wo > kMergeMax || count < 0 || ldg < wo) return record(QT_ERR_ARG);
     if (!G || !Tp || (!T && !hi) || (hi && (!lo || !exp_out || ldp < wo))) return record(QT_ERR_ARG);
     if (count == 0) return record(QT_OK);
-    constexpr size_t smem = sizeof(float) * (2 * kMergeMax * (kMergeMax + 1) + 96 * (kPanel + 1) + kPanel * (kPanel + 1));
+    constexpr size_t smem = sizeof(float) * (2 * kMergeMax * kMergeP + 32);
     static PerDeviceOnce attr_set;
     const int dev = current_device();
     if (attr_set.pending(dev)) {

@@ -116,3 +116,30 @@ def test_orders_beyond_the_panel_kernel_fall_back_with_a_warning(native_lib):
     with pytest.warns(UserWarning, match="torch.linalg.qr"):
         Q = _qr.householder_q(X.clone())
     assert float((Q - torch.linalg.qr(X).Q).abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("w", [1, 31, 33, 64, 72, 104, 128])
+def test_block_triangular_factor(native_lib, w):
+    """qt_merge_t against the column recurrence in float64: widths of one to four panels, ragged last panels."""
+    g = torch.Generator(device="cuda").manual_seed(w)
+    V = torch.tril(torch.randn(3, 300, w, device="cuda", dtype=torch.float64, generator=g) * 0.05, -1)
+    V[:, range(w), range(w)] = 1
+    tau, G = 2 / (V * V).sum(1), V.mT @ V
+
+    def factor(a, b):
+        T = torch.zeros(3, b - a, b - a, device="cuda", dtype=torch.float64)
+        for i in range(a, b):
+            T[:, i - a, i - a] = tau[:, i]
+            T[:, : i - a, i - a] = -tau[:, i, None] * (T[:, : i - a, : i - a] @ G[:, a:i, i:i + 1])[:, :, 0]
+        return T
+
+    Tp = torch.zeros(3, (w + 31) // 32, 32, 32, device="cuda")
+    for k in range(Tp.shape[1]):
+        t = factor(32 * k, min(w, 32 * k + 32))
+        Tp[:, k, : t.shape[1], : t.shape[2]] = t.float()
+    Gf, T = G.float().contiguous(), torch.full((3, w, w), 7.0, device="cuda")
+    rc = native_lib.qt_merge_t(Gf.data_ptr(), w, w * w, Tp.data_ptr(), Tp.stride(0), w, 3, T.data_ptr(), w * w,
+                               torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    ref = factor(0, w)
+    assert float((T.double() - ref).norm() / ref.norm()) < 5e-7
