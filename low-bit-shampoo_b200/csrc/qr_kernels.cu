@@ -862,7 +862,7 @@ int launch_householder_panel(float *A, long long strideA, int n, int ld, int cou
 // below the diagonal blocks).  Bound by latency and by shared-memory wavefronts: the chain is two products of 32^3 and two of
 // 64^3 where panel after panel took three pairs of products that grew with the columns done, and a warp's tile of 8 rows
 // x 16 columns reads four k of a row and of four columns at a time, conflict-free: 5 wavefronts per 4 x 128
-// multiply-adds (one operand and one wavefront per multiply-add before).  27 -> 12 us.
+// multiply-adds (one operand and one wavefront per multiply-add before).  28 -> 14 us.
 static constexpr int kMergeMax = 128, kMergeP = 132;         // row pitch: 16-byte rows, 8 rows meet 32 banks
 
 // out[i][j] (+)= sgn * sum over l in [l0, l1) of A[i][l] B[l][j], for this lane's row i and columns j .. j+3
