@@ -41,6 +41,7 @@ struct GemmExtras {
     int max_ctas = 0;                                       // > 0: cap of the persistent grid (SMs left to kernels on other streams)
     int c_follows_d = 0;                                    // C indexed through d_slot like the outputs
     int sym = 0;                                            // the result is symmetric (M == N): tiles on and above the diagonal, mirrored
+    int chained = 0;                                        // the launch may overlap the end of its predecessor (see launch_chained)
     float *amax_out = nullptr;                              // per output entry: max |result| (atomic max; zeroed by the caller)
     float *cd_part = nullptr;                               // column sums of result * C instead of a stored result: per matrix
                                                             // [4 * ceil(M / 128)][N] partial sums (two planes)

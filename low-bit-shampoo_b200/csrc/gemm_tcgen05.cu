@@ -448,6 +448,7 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    chain_wait();
     __syncthreads();
     if constexpr (PAIR) cluster_sync_all();                   // the peer's barriers are initialised, its tensor memory allocated
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -531,6 +532,7 @@ k_gemm_bf16x3(const __grid_constant__ GemmMaps maps, const GemmParams p) {
                     }
                 }
             }
+            chain_release();                                  // every load of this CTA is on its way: one tile's products and epilogue remain
         }
     } else if (warp == EPI_WARPS + 1) {
         // ---------------- MMA issuer: accumulator j % NACC in TMEM columns [ (j % NACC) * BN_, +BN_ )
@@ -1442,7 +1444,7 @@ int launch_gemm_planes(const GemmArgs &a, const void *Amid, const void *Bmid, cu
     }
     unsigned grid = (unsigned)(ctas < sms ? ctas : sms);                         // persistent: one CTA per SM
     if (x.max_ctas > 0 && grid > (unsigned)x.max_ctas) grid = (unsigned)x.max_ctas;
-    kern<<<grid, g_cfg_threads[cfg], GEMM_SMEM, s>>>(maps, p);
+    if (launch_chained(kern, grid, g_cfg_threads[cfg], GEMM_SMEM, s, x.chained != 0, maps, p) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
     count_launch(1);
     return check_launch();
 }

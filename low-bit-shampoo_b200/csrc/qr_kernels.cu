@@ -398,6 +398,7 @@ __global__ void __launch_bounds__(kPt, 1)
 k_panel(float *__restrict__ Abase, long long strideA, int n, int ld, int j0, int w, float *__restrict__ Vbase, long long strideV,
         float *__restrict__ Tbase, long long strideT, int prev_w, const float *__restrict__ Tprev_base, int block_end, const PanelPlanes planes) {
     extern __shared__ float sm[];
+    chain_wait();
     const int m = n - j0;
     float *Pall = sm;                                      // [32 + 32 RT + 32][33]: window rows above the panel, panel rows, zeros
     float *P = Pall + kPanel * kPp;
@@ -581,6 +582,7 @@ k_panel(float *__restrict__ Abase, long long strideA, int n, int ld, int j0, int
         }
         __syncthreads();
         if (chunk > 0) {                                   // not the new panel: write the updated chunk back and leave
+            chain_release();
 #pragma unroll 4
             for (int r = warp; r < mu; r += kPw)
                 if (lane < wc) Cg[(long long)r * ld + lane] = C[r * kPp + lane];
@@ -728,6 +730,7 @@ k_panel(float *__restrict__ Abase, long long strideA, int n, int ld, int j0, int
         }
         if (next) asm volatile("bar.arrive 3, 512;" ::: "memory");
     }
+    chain_release();
     __syncthreads();
     // ---- triangular factor from V^T V and tau (LAPACK slarft): four 8 x 8 blocks, then -T1 (G12 T2) for the off-diagonal
     // blocks of 8 and of 16.  Eight warps; the others store V meanwhile.  (One warp running down 32 columns took 5600 clocks.)
@@ -787,7 +790,7 @@ k_panel(float *__restrict__ Abase, long long strideA, int n, int ld, int j0, int
 
 template <int RT>
 static int launch_panel(float *A, long long strideA, int n, int ld, int count, int j0, int w, float *V, long long strideV, float *T, long long strideT,
-                        cudaStream_t s, int prev_w, const float *Tprev, int block_end, const PanelPlanes &planes) {
+                        cudaStream_t s, int prev_w, const float *Tprev, int block_end, const PanelPlanes &planes, bool chained) {
     const size_t smem = sizeof(float) * ((size_t)(32 * RT + 64) * kPp + 8 * 32 * 33 + 5 * 32 * 33 + 32);
     static PerDeviceOnce attr_set;
     const int dev = current_device();
@@ -796,7 +799,8 @@ static int launch_panel(float *A, long long strideA, int n, int ld, int count, i
         attr_set.mark(dev);
     }
     const int chunks = prev_w > 0 ? (block_end - j0 + kPanel - 1) / kPanel : 1;
-    k_panel<RT><<<dim3(count, chunks), kPt, smem, s>>>(A, strideA, n, ld, j0, w, V, strideV, T, strideT, prev_w, Tprev, block_end, planes);
+    if (launch_chained(k_panel<RT>, dim3(count, chunks), kPt, smem, s, chained, A, strideA, n, ld, j0, w, V, strideV, T, strideT, prev_w, Tprev, block_end,
+                       planes) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
     count_launch(1);
     return check_launch();
 }
@@ -826,7 +830,7 @@ static int launch_panel_rpl(float *A, long long strideA, int n, int ld, int coun
 int launch_householder_panel(float *A, long long strideA, int n, int ld, int count, int j0, int w,
                              float *V, long long strideV, float *T, long long strideT, cudaStream_t s,
                              int prev_w, const float *Tprev, int block_end,
-                             void *planes_hi, void *planes_lo, long long ldp, long long strideP, int plane_col, int rows_above, int plane_exp) {
+                             void *planes_hi, void *planes_lo, long long ldp, long long strideP, int plane_col, int rows_above, int plane_exp, bool chained) {
     const PanelPlanes planes{static_cast<__half *>(planes_hi), static_cast<__half *>(planes_lo), ldp, strideP, plane_col, rows_above,
                              ldexpf(1.0f, plane_exp)};
     if (ld < n || n <= 0 || count < 0 || j0 < 0 || j0 >= n || w <= 0 || w > kPanel || j0 + w > n) return record(QT_ERR_ARG);
@@ -843,15 +847,15 @@ int launch_householder_panel(float *A, long long strideA, int n, int ld, int cou
         return launch_panel_rpl<24, 14>(QT_ARGS);
     }
     // rows per lane are rounded up to a multiple of four: the factorisation's time goes with them
-    if (rows_per_lane <= 4) return launch_panel<4>(QT_ARGS);
-    if (rows_per_lane <= 8) return launch_panel<8>(QT_ARGS);
-    if (rows_per_lane <= 12) return launch_panel<12>(QT_ARGS);
-    if (rows_per_lane <= 16) return launch_panel<16>(QT_ARGS);
-    if (rows_per_lane <= 20) return launch_panel<20>(QT_ARGS);
-    if (rows_per_lane <= 24) return launch_panel<24>(QT_ARGS);
-    if (rows_per_lane <= 28) return launch_panel<28>(QT_ARGS);
-    if (rows_per_lane <= 32) return launch_panel<32>(QT_ARGS);
-    return launch_panel<38>(QT_ARGS);
+    if (rows_per_lane <= 4) return launch_panel<4>(QT_ARGS, chained);
+    if (rows_per_lane <= 8) return launch_panel<8>(QT_ARGS, chained);
+    if (rows_per_lane <= 12) return launch_panel<12>(QT_ARGS, chained);
+    if (rows_per_lane <= 16) return launch_panel<16>(QT_ARGS, chained);
+    if (rows_per_lane <= 20) return launch_panel<20>(QT_ARGS, chained);
+    if (rows_per_lane <= 24) return launch_panel<24>(QT_ARGS, chained);
+    if (rows_per_lane <= 28) return launch_panel<28>(QT_ARGS, chained);
+    if (rows_per_lane <= 32) return launch_panel<32>(QT_ARGS, chained);
+    return launch_panel<38>(QT_ARGS, chained);
 #undef QT_ARGS
 }
 
@@ -887,6 +891,7 @@ k_merge_t(const float *__restrict__ Gbase, long long ldg, long long strideG,
           float *__restrict__ Tbase, long long strideT,
           __half *__restrict__ hi, __half *__restrict__ lo, long long ldp, long long strideP, int *__restrict__ exp_out, int target) {
     extern __shared__ __align__(16) float merge_sm[];
+    chain_wait();
     float *Ts = merge_sm, *Gs = Ts + kMergeMax * kMergeP, *red = Gs + kMergeMax * kMergeP;
     const float *G = Gbase + (long long)blockIdx.x * strideG;
     const float *Tp = Tp_base + (long long)blockIdx.x * strideTp;
@@ -929,6 +934,7 @@ k_merge_t(const float *__restrict__ Gbase, long long ldg, long long strideG,
         *reinterpret_cast<float4 *>(Ts + (b + i1) * kMergeP + b + 32 + j1) = make_float4(-r.x, -r.y, -r.z, -r.w);
     }
     __syncthreads();
+    chain_release();
     if (wo > 64) {                                            // the pair of 64: all warps
         const int i2 = 8 * (warp & 7) + (lane >> 2), j2 = 16 * (warp >> 3) + 4 * (lane & 3);
         *reinterpret_cast<float4 *>(Gs + (64 + i2) * kMergeP + j2) = merge_dot(Gs + i2 * kMergeP + 64, Ts + 64 * kMergeP + 64 + j2, 0, 16 * (warp >> 3) + 16);
@@ -993,7 +999,7 @@ k_merge_t(const float *__restrict__ Gbase, long long ldg, long long strideG,
 }
 
 int launch_merge_t(const float *G, long long ldg, long long strideG, const float *Tp, long long strideTp, int wo, int count,
-                   float *T, long long strideT, cudaStream_t s, void *hi, void *lo, long long ldp, long long strideP, int *exp_out, int target) {
+                   float *T, long long strideT, cudaStream_t s, void *hi, void *lo, long long ldp, long long strideP, int *exp_out, int target, bool chained) {
     if (wo <= 0 || wo > kMergeMax || count < 0 || ldg < wo) return record(QT_ERR_ARG);
     if (!G || !Tp || (!T && !hi) || (hi && (!lo || !exp_out || ldp < wo))) return record(QT_ERR_ARG);
     if (count == 0) return record(QT_OK);
@@ -1005,8 +1011,8 @@ int launch_merge_t(const float *G, long long ldg, long long strideG, const float
             return record(QT_ERR_LAUNCH);
         attr_set.mark(dev);
     }
-    k_merge_t<<<count, 1024, smem, s>>>(G, ldg, strideG, Tp, strideTp, wo, T, strideT, static_cast<__half *>(hi), static_cast<__half *>(lo), ldp,
-                                        strideP, exp_out, target);
+    if (launch_chained(k_merge_t, count, 1024, smem, s, chained, G, ldg, strideG, Tp, strideTp, wo, T, strideT, static_cast<__half *>(hi),
+                       static_cast<__half *>(lo), ldp, strideP, exp_out, target) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
     count_launch(1);
     return check_launch();
 }

@@ -50,13 +50,32 @@ struct DequantArgs {
     void *out; int out_dtype; long long stride_out;         // elements
 };
 
+// Launches of one chain on a stream (programmatic dependent launch): with `chained` the kernel may be brought onto the
+// chip while its predecessor ends.  It calls chain_wait() before its first access to global memory - which returns when
+// the predecessor is complete and its writes are visible, at once without the attribute - and chain_release() when its
+// remaining work is short, so that a waiting successor does not hold SMs that other streams could use.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool chained, A... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cfg.attrs = attr; cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 int launch_grad_planes(const void *stat_items, int n_stat, const void *split_items, int n_split, const long long *grads, float *part_amax,
                        float *part_ss, int *gexp, int target, void *plane_base, cudaStream_t stream);
 int read_apply_error(bool clear);    // error words of the kernels in apply_kernels.cu and refresh.cu
 int read_refresh_error(bool clear);
 int launch_merge_t(const float *G, long long ldg, long long strideG, const float *Tp, long long strideTp, int wo, int count,
                    float *T, long long strideT, cudaStream_t stream, void *hi = nullptr, void *lo = nullptr, long long ldp = 0,
-                   long long strideP = 0, int *exp_out = nullptr, int target = 0);
+                   long long strideP = 0, int *exp_out = nullptr, int target = 0, bool chained = false);
 int launch_quantize(const QuantArgs &a, cudaStream_t stream);
 int launch_dequantize(const DequantArgs &a, cudaStream_t stream);
 // a.out / a.out_dtype / a.stride_out are ignored: output goes to the bf16 planes hi, lo
@@ -74,6 +93,6 @@ int launch_householder_panel(float *A, long long strideA, int n, int ld, int cou
                              int prev_w = 0, const float *Tprev = nullptr, int block_end = 0,
                              // scaled fp16 planes of V (see qr_kernels.cu); null: none
                              void *planes_hi = nullptr, void *planes_lo = nullptr, long long ldp = 0, long long strideP = 0,
-                             int plane_col = 0, int rows_above = 0, int plane_exp = 0);
+                             int plane_col = 0, int rows_above = 0, int plane_exp = 0, bool chained = false);
 
 }  // namespace qt

@@ -108,6 +108,7 @@ struct RowPlanes { __half *hi, *lo; const float *scale, *amax; int *exp_out; int
 __global__ void __launch_bounds__(kThreadsR)
 k_rows_to_planes(const float *__restrict__ X, long long ldx, long long strideX, int rows, int cols, const long long *__restrict__ index,
                  long long stride_index, long long stride_scale, long long ldp, long long strideP, const RowPlanes a, const RowPlanes b, int target) {
+    chain_wait();
     const int m = blockIdx.y;
     const float *x = X + (long long)m * strideX;
     const long long *idx = index ? index + (long long)m * stride_index : nullptr;
@@ -155,6 +156,7 @@ k_rows_to_planes(const float *__restrict__ X, long long ldx, long long strideX, 
 // Q = I, fp32 and planes.
 __global__ void __launch_bounds__(kThreadsR)
 k_identity(float *__restrict__ X, long long ldx, __half *__restrict__ hi, __half *__restrict__ lo, int n, long long ldp, long long strideP, float scale) {
+    chain_wait();
     float *x = X + (long long)blockIdx.y * n * ldx;
     hi += (long long)blockIdx.y * strideP;
     lo += (long long)blockIdx.y * strideP;
@@ -341,12 +343,23 @@ struct Bump {
 // alpha op(A) op(B) + beta C: into D and / or the planes P (exponents as P says; `rel`: worst-case exponents, written to P.exp).
 struct Out { float *D = nullptr; long long ldd = 0, strideD = 0; const P2 *P = nullptr; bool rel = false; const float *C = nullptr; float alpha = 1.0f, beta = 0.0f;
              int sym = 0; float *amax = nullptr; const int *slot = nullptr; float *cd = nullptr; };
-static int product(const P2 &A, bool ta, const P2 &B, bool tb, int M, int N, int K, int batch, const Out &o, cudaStream_t s) {
+// The stream of a pass.  In a small class the next kernel is brought onto the chip while its predecessor ends (see
+// launch_chained): some 150 launches of 10 to 60 us follow each other, and start-up and prologue are 2 us of each (8
+// matrices of 1000 and 8 of 512: 3.55 -> 3.35 ms, 4 of 1189 and 4 of 777: 3.90 -> 3.70).  Where a product has several
+// rounds of tiles the kernels are long, and waiting ones hold SMs that other classes would use (ViT-B/32: 24.3 -> 24.8 ms).
+struct Queue {
+    cudaStream_t stream;
+    bool chained;
+    operator cudaStream_t() const { return stream; }
+};
+
+static int product(const P2 &A, bool ta, const P2 &B, bool tb, int M, int N, int K, int batch, const Out &o, const Queue &s) {
     GemmArgs a{A.hi, A.lo, A.ld, A.stride, ta ? 1 : 0, B.hi, B.lo, B.ld, B.stride, tb ? 0 : 1, M, N, K, batch, o.alpha, o.beta,
                o.C, o.ldd, o.strideD, o.D, o.ldd, o.strideD, o.P ? o.P->hi : nullptr, o.P ? o.P->lo : nullptr, o.P ? o.P->ld : 0, o.P ? o.P->stride : 0};
     GemmExtras x;
     x.f16 = 1; x.kc = 2; x.a_exp = A.exp; x.b_exp = B.exp; x.ab_exp0 = A.exp0 + B.exp0;
     x.sym = o.sym; x.amax_out = o.amax; x.cd_part = o.cd;
+    x.chained = s.chained;                                    // a product is never the first launch of a pass
     if (o.slot) { x.d_slot = o.slot; x.c_follows_d = 1; }
     if (o.P) {
         if (o.rel) { x.out_rel = 1; x.out_exp0 = kMaxExp - ceil_log2(K) - A.tmax - B.tmax; x.out_exp_w = o.P->exp; }
@@ -364,11 +377,11 @@ static dim3 rows_grid(long long threads, int m) {
 
 static int to_planes(const float *X, long long ldx, long long strideX, int rows, int cols, int m, const long long *index, long long stride_index,
                      long long stride_scale, const P2 &a, const float *scale_a, const float *amax_a, const P2 *b, const float *scale_b,
-                     const float *amax_b, cudaStream_t s) {
+                     const float *amax_b, const Queue &s) {
     RowPlanes ra{a.hi, a.lo, scale_a, amax_a, amax_a ? a.exp : nullptr, a.exp0}, rb{nullptr, nullptr, nullptr, nullptr, nullptr, 0};
     if (b) rb = RowPlanes{b->hi, b->lo, scale_b, amax_b, amax_b ? b->exp : nullptr, b->exp0};
-    k_rows_to_planes<<<rows_grid((long long)rows * ((cols + 7) / 8), m), kThreadsR, 0, s>>>(X, ldx, strideX, rows, cols, index, stride_index, stride_scale,
-                                                                                         a.ld, a.stride, ra, rb, kTarget);
+    if (launch_chained(k_rows_to_planes, rows_grid((long long)rows * ((cols + 7) / 8), m), kThreadsR, 0, s, s.chained, X, ldx, strideX, rows, cols, index, stride_index, stride_scale,
+                       a.ld, a.stride, ra, rb, kTarget) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
     count_launch(1);
     return check_launch();
 }
@@ -406,7 +419,7 @@ static void qr_space(Bump &w, int m, int n, QrSpace &q) {
     q.Pw = w.planes(m, kOuter, n, 0, w.of<int>(m));
     q.Py.tmax = q.Pw.tmax = kMaxExp;
 }
-static int qr_batch(int m, int n, float *X, const P2 &Px, float *Q, const P2 &Pq, QrSpace &q, cudaStream_t s) {
+static int qr_batch(int m, int n, float *X, const P2 &Px, float *Q, const P2 &Pq, QrSpace &q, const Queue &s) {
     const long long ld = q.ld, nn = n * ld;                   // fp32 matrices have rows of a multiple of 32 bytes
     const int npan = (n + kPan - 1) / kPan;
     auto block = [&](int J0, P2 &pv, P2 &pt) {
@@ -436,16 +449,17 @@ static int qr_batch(int m, int n, float *X, const P2 &Px, float *Q, const P2 &Pq
             const int w = J0 + wo - j0 < kPan ? J0 + wo - j0 : kPan, k = j0 / kPan, prev = j0 > J0 ? kPan : 0;
             QT_TRY(launch_householder_panel(X, nn, n, (int)ld, m, j0, w, q.V, nn, q.T + (long long)k * kPan * kPan, (long long)npan * kPan * kPan, s,
                                             prev, prev ? q.T + (long long)(k - 1) * kPan * kPan : nullptr, J0 + wo,
-                                            pv.hi, pv.lo, pv.ld, pv.stride, j0 - J0, j0 - J0, kBasisExp));
+                                            pv.hi, pv.lo, pv.ld, pv.stride, j0 - J0, j0 - J0, kBasisExp, s.chained));
         }
         Out og; og.D = q.G; og.ldd = wo; og.strideD = (long long)wo * wo; og.sym = 1;
         QT_TRY(product(pv, true, pv, false, wo, wo, n - J0, m, og, s));
         QT_TRY(launch_merge_t(q.G, wo, (long long)wo * wo, q.T + (long long)(J0 / kPan) * kPan * kPan, (long long)npan * kPan * kPan, wo, m, nullptr, 0, s,
-                              pt.hi, pt.lo, pt.ld, pt.stride, pt.exp, kTarget));
+                              pt.hi, pt.lo, pt.ld, pt.stride, pt.exp, kTarget, s.chained));
         const int rows = n - J0, t = rows - wo;
         if (t > 0) QT_TRY(reflect(pv, pt, true, wo, rows, t, X + J0 * ld + J0 + wo, Px.window(J0, J0 + wo)));
     }
-    k_identity<<<rows_grid((long long)n * (Pq.ld / 2), m), kThreadsR, 0, s>>>(Q, ld, Pq.hi, Pq.lo, n, Pq.ld, Pq.stride, ldexpf(1.0f, kBasisExp));
+    if (launch_chained(k_identity, rows_grid((long long)n * (Pq.ld / 2), m), kThreadsR, 0, s, s.chained, Q, ld, Pq.hi, Pq.lo, n, Pq.ld, Pq.stride,
+                       ldexpf(1.0f, kBasisExp)) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
     count_launch(1);
     for (int J0 = (n - 1) / kOuter * kOuter; J0 >= 0; J0 -= kOuter) {
         const int wo = block(J0, pv, pt), rows = n - J0;
@@ -455,10 +469,11 @@ static int qr_batch(int m, int n, float *X, const P2 &Px, float *Q, const P2 &Pq
 }
 
 // One pass over matrices a .. a+m-1 of the class; with w.base == nullptr only the workspace is measured.
-static int refresh_pass(const qt_refresh_desc &d, int a, int m, Bump &w, bool run, cudaStream_t s) {
+static int refresh_pass(const qt_refresh_desc &d, int a, int m, Bump &w, bool run, cudaStream_t stream) {
     const int n = d.n, keep = d.keep, nb = (n + d.blocksize - 1) / d.blocksize;
     const long long ld = up(n, 8), nn = n * ld;               // fp32 scratch matrices have rows of a multiple of 32 bytes
     const int tiles = (n + 127) / 128;
+    const Queue s{stream, (long long)tiles * tiles * m <= 4LL * device_sm_count()};
     float *weights = w.of<float>((long long)m * keep), *bound = w.of<float>(m), *amax = w.of<float>(2 * m);
     int *exps = w.of<int>(4 * m);
     float *S = d.S + (long long)a * keep, *max_eig = d.max_eig + a;
