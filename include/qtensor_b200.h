@@ -504,7 +504,7 @@ int qt_column_dot(const float *A, const float *B, long long ld, long long stride
 #define QT_APPLY_GROUP_BYTES 640
 typedef struct qt_apply_wave {
     const void *plane_items; const void *groups1, *groups2; const int *tiles1, *tiles2;
-    int n_plane_items, n_groups, n_tiles1, n_tiles2, bn, reserved;
+    int n_plane_items, n_groups, n_tiles1, n_tiles2, bn1, bn2;   /* bn: tile width of each product, as its groups were filled */
 } qt_apply_wave;
 typedef struct qt_apply_desc {
     const void *stat_items; const qt_apply_wave *waves; const long long *grads; const float *code;

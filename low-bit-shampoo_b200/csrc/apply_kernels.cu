@@ -309,7 +309,11 @@ template <int BN> struct ApplyCfg {
     static constexpr int BM = 128, BK = 64, KC = 2;
     static constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
     static constexpr int STAGE = 2 * (A_BYTES + B_BYTES), STAGES = 12 * A_BYTES / STAGE;
-    static constexpr int EC = BN / 2, EPI = 8, THREADS = (EPI + 2) * 32, NACC = 512 / BN;
+    static constexpr int EC = BN / 2, EPI = 8, NACC = 512 / BN;
+    // 128 partial sums a thread need more than the 168 registers that ten warps get: two idle warps complete the producers'
+    // warpgroup, which hands registers to the epilogue (launch: 384 x 168 = 256 x 224 + 128 x 56)
+    static constexpr bool REGS = BN == 256;
+    static constexpr int THREADS = (EPI + (REGS ? 4 : 2)) * 32;
     static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
 };
 static constexpr int kMaxGroups = 256;
@@ -332,7 +336,8 @@ k_apply_gemm(const ApplyGroup *__restrict__ groups, const int *__restrict__ tile
     auto acc_full = [&](int a) { return bar0 + 8u * (2 * STAGES + a); };
     auto acc_empty = [&](int a) { return bar0 + 8u * (2 * STAGES + NACC + a); };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (*reinterpret_cast<volatile int *>(&g_gemm_error) == QT_ERR_TIMEOUT) return;   // an earlier wait expired: drain fast
+    // an earlier wait expired: drain fast (all threads or none, the epilogue waits for registers)
+    if (__syncthreads_or(*reinterpret_cast<volatile int *>(&g_gemm_error) == QT_ERR_TIMEOUT)) return;
     for (int i = threadIdx.x; i <= ngroups; i += Cfg::THREADS) starts[i] = tile_start[i];
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
@@ -350,6 +355,8 @@ k_apply_gemm(const ApplyGroup *__restrict__ groups, const int *__restrict__ tile
     const unsigned tmem_base = *tmem_slot;
     const int num_tiles = starts[ngroups];
 
+    if (warp >= EPI) {
+    if constexpr (Cfg::REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == EPI) {
         if (lane == 0) {                                      // TMA producer
             unsigned it = 0;
@@ -424,7 +431,9 @@ k_apply_gemm(const ApplyGroup *__restrict__ groups, const int *__restrict__ tile
                 }
             }
         }
+    }
     } else {                                                  // epilogue: warp e holds rows 32 (e & 3) .., columns EC (e >> 2) ..
+        if constexpr (Cfg::REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
         const int quad = warp & 3, seg = warp >> 2;
         int j = 0, gi = 0;
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
@@ -623,7 +632,8 @@ static bool prepare_apply() {
     const int dev = current_device();
     if (done.pending(dev)) {
         if (cudaFuncSetAttribute(k_apply_gemm<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, ApplyCfg<128>::SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_apply_gemm<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, ApplyCfg<192>::SMEM) != cudaSuccess)
+            cudaFuncSetAttribute(k_apply_gemm<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, ApplyCfg<192>::SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_apply_gemm<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, ApplyCfg<256>::SMEM) != cudaSuccess)
             return false;
         done.mark(dev);
     }
@@ -633,7 +643,9 @@ static bool prepare_apply() {
 static void launch_apply_gemm(const void *groups, const int *tiles, int ngroups, int ntiles, int bn, cudaStream_t s) {
     const int sms = device_sm_count();
     const unsigned grid = (unsigned)(ntiles < sms ? ntiles : sms);
-    if (bn == 192)
+    if (bn == 256)
+        k_apply_gemm<256><<<grid, ApplyCfg<256>::THREADS, ApplyCfg<256>::SMEM, s>>>(static_cast<const ApplyGroup *>(groups), tiles, ngroups);
+    else if (bn == 192)
         k_apply_gemm<192><<<grid, ApplyCfg<192>::THREADS, ApplyCfg<192>::SMEM, s>>>(static_cast<const ApplyGroup *>(groups), tiles, ngroups);
     else
         k_apply_gemm<128><<<grid, ApplyCfg<128>::THREADS, ApplyCfg<128>::SMEM, s>>>(static_cast<const ApplyGroup *>(groups), tiles, ngroups);
@@ -661,7 +673,7 @@ int qt_apply_group(void *out, const void *Ahi, const void *Alo, long long lda, l
                    const int *a_exp, const int *b_exp, void *Phi, void *Plo, long long ldp, long long strideP, int *out_exp, int rel,
                    void *D, long long ldd, int wide, float *part) {
     static_assert(sizeof(ApplyGroup) == QT_APPLY_GROUP_BYTES && sizeof(ApplyItem) == 80 && sizeof(ApplyTensor) == 72, "table layouts");
-    if (!out || !Ahi || !Alo || !Bhi || !Blo || M <= 0 || N <= 0 || K <= 0 || batch <= 0 || (bn != 128 && bn != 192)) return record(QT_ERR_ARG);
+    if (!out || !Ahi || !Alo || !Bhi || !Blo || M <= 0 || N <= 0 || K <= 0 || batch <= 0 || (bn != 128 && bn != 192 && bn != 256)) return record(QT_ERR_ARG);
     if (lda % 8 || ldb % 8 || strideA % 8 || strideB % 8 || !a_exp || !b_exp || (!Phi && (!D || !part)) || (Phi && (!Plo || !out_exp || ldp % 16)))
         return record(QT_ERR_ARG);
     ApplyGroup g;
@@ -697,8 +709,8 @@ int qt_apply_run(const qt_apply_desc *d, void *stream) {
             count_launch(1);
         }
         if (v.n_groups > 0) {
-            launch_apply_gemm(v.groups1, v.tiles1, v.n_groups, v.n_tiles1, v.bn, s);
-            launch_apply_gemm(v.groups2, v.tiles2, v.n_groups, v.n_tiles2, v.bn, s);
+            launch_apply_gemm(v.groups1, v.tiles1, v.n_groups, v.n_tiles1, v.bn1, s);
+            launch_apply_gemm(v.groups2, v.tiles2, v.n_groups, v.n_tiles2, v.bn2, s);
         }
     }
     if (d->n_chunks > 0) {

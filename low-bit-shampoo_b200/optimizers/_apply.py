@@ -37,7 +37,7 @@ GROUP_BYTES = 640               # the stride of the groups in device memory (inc
 class Wave(ct.Structure):
     _fields_ = [("plane_items", ct.c_void_p), ("groups1", ct.c_void_p), ("groups2", ct.c_void_p), ("tiles1", ct.c_void_p),
                 ("tiles2", ct.c_void_p), ("n_plane_items", ct.c_int), ("n_groups", ct.c_int), ("n_tiles1", ct.c_int),
-                ("n_tiles2", ct.c_int), ("bn", ct.c_int), ("reserved", ct.c_int)]
+                ("n_tiles2", ct.c_int), ("bn1", ct.c_int), ("bn2", ct.c_int)]
 
 
 class Desc(ct.Structure):
@@ -74,6 +74,22 @@ class PointerTable:
 
 class _Block:
     __slots__ = ("param", "r0", "c0", "m", "k", "s0", "s1", "stat", "index")
+
+
+def _tile_width(waves, sms):
+    """Tile width of one product of all blocks; waves: lists of (rows, columns, K, blocks).  A tile's time is linear in
+    K: operand delivery from L2 per k - wider tiles need less of it per result - and the part of its epilogue that the next
+    tile's products do not hide.  Tiles go to the SMs in turn, so a plan's time is the longest sum over an SM.  Microseconds of
+    both products, 128 / 192 / 256: ViT-B/32 905 / 891 / 849, ResNet-34 215 / 225 / 208, 8 x (512 x 1000) 52 / 65 / 56."""
+    def cost(width, per_k, fixed):
+        total = 0.0
+        for groups in waves:
+            times = np.concatenate([np.full(math.ceil(m / 128) * math.ceil(n / width) * count, per_k * k + fixed) for m, n, k, count in groups])
+            total += np.pad(times, (0, -len(times) % sms)).reshape(-1, sms).sum(0).max()
+        return total
+    if not waves:
+        return 128
+    return min(((cost(w, *c), w) for w, c in ((128, (0.0147, 1.0)), (192, (0.0174, 1.9)), (256, (0.0215, 3.5)))))[1]
 
 
 def _up(x, q):
@@ -193,9 +209,9 @@ class ApplyPlan:
         self._keep.append(ints)
         exp = lambda kind_, i: ints.data_ptr() + 4 * (kind_ * tc + i)
 
-        # tiles of 192 columns pay once they fill the chip more than once; below that the narrower ones spread better
-        tiles = lambda bn: sum(math.ceil(m / 128) * math.ceil(k / bn) * len(bs) for w in waves for m, k, bs in w)
-        bn = 192 if tiles(192) >= 2 * torch.cuda.get_device_properties(dev).multi_processor_count else 128
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        bn1 = _tile_width([[(m, k, m, len(bs)) for m, k, bs in w] for w in waves], sms)
+        bn2 = _tile_width([[(m, k, k, len(bs)) for m, k, bs in w] for w in waves], sms)
 
         # ---- work items and groups of every wave
         ranges = defaultdict(list)                            # per parameter: pieces of the direction's sum of squares
@@ -210,7 +226,7 @@ class ApplyPlan:
                 for rows, ld in ((m, lm), (k, lk), (m, lk), (m, lk)):          # P0, P1, G, T
                     regions.append((cursor, cursor + _up(n * rows * ld, 64)))
                     cursor += 2 * _up(n * rows * ld, 64)
-                nt = math.ceil(m / 128) * math.ceil(k / bn)
+                nt = math.ceil(m / 128) * math.ceil(k / bn2)
                 for j, b in enumerate(bs):
                     b.index = index + j
                     ranges[b.param].append((parts + 8 * nt * j, 8 * nt))
@@ -272,18 +288,18 @@ class ApplyPlan:
                                           wb + 2 * regions[side][0] + at, wb + 2 * regions[side][1] + at))
                 dp = torch.tensor(dptrs, dtype=torch.int64).to(dev)
                 self._keep.append(dp)
-                nt = math.ceil(m / 128) * math.ceil(k / bn) * n
+                count = lambda bn: math.ceil(m / 128) * math.ceil(k / bn) * n
                 rel = _gemm.F16_MAX_EXP - _gemm._ceil_log2(m) - 2 * _gemm.SPLIT_TARGET
                 at = lambda q, h: wb + 2 * regions[q][h]
-                for lst, tl, args in (
-                        (g1, t1, (at(0, 0), at(0, 1), lm, m * lm, at(2, 0), at(2, 1), lk, m * lk, m, k, m, n, bn, t1[-1], exp(0, i0), exp(2, i0),
+                for lst, tl, bn, args in (
+                        (g1, t1, bn1, (at(0, 0), at(0, 1), lm, m * lm, at(2, 0), at(2, 1), lk, m * lk, m, k, m, n, bn1, t1[-1], exp(0, i0), exp(2, i0),
                                   at(3, 0), at(3, 1), lk, m * lk, exp(3, i0), rel, None, 0, 0, None)),
-                        (g2, t2, (at(3, 0), at(3, 1), lk, m * lk, at(1, 0), at(1, 1), lk, k * lk, m, k, k, n, bn, t2[-1], exp(3, i0), exp(1, i0),
+                        (g2, t2, bn2, (at(3, 0), at(3, 1), lk, m * lk, at(1, 0), at(1, 1), lk, k * lk, m, k, k, n, bn2, t2[-1], exp(3, i0), exp(1, i0),
                                   None, None, 0, 0, None, 0, dp.data_ptr(), widths[bs[0].param], wide, part(part0)))):
                     buf = ct.create_string_buffer(GROUP_BYTES)
                     F._check(lib.qt_apply_group(buf, *args), "apply group")
                     lst.append(buf.raw)
-                    tl.append(tl[-1] + nt)
+                    tl.append(tl[-1] + count(bn))
             wave_tables.append((items, g1, g2, t1, t2))
         if simt_second:
             if not wave_tables:
@@ -301,7 +317,7 @@ class ApplyPlan:
         self.waves = (Wave * max(1, len(wave_tables)))()
         for wv, (items, g1, g2, t1, t2) in zip(self.waves, wave_tables):
             wv.plane_items, wv.n_plane_items = up(table(items)), len(items)
-            wv.groups1, wv.groups2, wv.n_groups, wv.bn = up(b"".join(g1)), up(b"".join(g2)), len(g1), bn
+            wv.groups1, wv.groups2, wv.n_groups, wv.bn1, wv.bn2 = up(b"".join(g1)), up(b"".join(g2)), len(g1), bn1, bn2
             wv.tiles1, wv.tiles2 = up(np.array(t1, dtype=np.int32).tobytes()), up(np.array(t2, dtype=np.int32).tobytes())
             wv.n_tiles1, wv.n_tiles2 = t1[-1], t2[-1]
         total = sum(numels)

@@ -55,6 +55,18 @@ def test_waves_give_the_same_bits(native_lib):
     assert all(torch.equal(x, y) for x, y in zip(a, b))
 
 
+@pytest.mark.parametrize("width", [128, 192, 256])
+def test_tile_widths_agree(width, native_lib, monkeypatch):
+    """The width is chosen by size (_tile_width); only the order of a norm's partial sums depends on it."""
+    from optimizers import _apply
+    shapes = SHAPES + [(130, 257), (257, 130), (128, 449), (449, 64)]
+    a = run("adamw", shapes, True)
+    monkeypatch.setattr(_apply, "_tile_width", lambda waves, sms: width)
+    for x, y in zip(a, run("adamw", shapes, True)):
+        assert float((x - y).norm()) <= 1e-6 * float(y.norm())
+    assert native_lib.qt_device_error(1) == 0
+
+
 def test_gradients_that_move_and_graph_replay(native_lib):
     """Gradients at new addresses every step (above) and steps under cuda_graph=True give the eager results."""
     a, b = run("adamw", SHAPES, True), run("adamw", SHAPES, True, cuda_graph=True)
