@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(kThreadsR)
 k_basis_rows(const unsigned char *__restrict__ codes, long long stride_codes, const float *__restrict__ absmax_base, long long stride_absmax,
              const float *__restrict__ code, int n, int nb, int bs_shift, const long long *__restrict__ index, long long stride_index, int rows,
              float *__restrict__ X, long long ldx, long long strideX, __half *__restrict__ hi, __half *__restrict__ lo, long long ldp, long long strideP, float scale) {
+    chain_wait();
     __shared__ float2 pair_lut[BITS == 4 ? 256 : 1];
     __shared__ float code_s[BITS == 8 ? 256 : 1];
     if constexpr (BITS == 4) pair_lut[threadIdx.x] = make_float2(__ldg(code + (threadIdx.x >> 4)), __ldg(code + (threadIdx.x & 15)));
@@ -175,6 +176,7 @@ k_identity(float *__restrict__ X, long long ldx, __half *__restrict__ hi, __half
 // order), sorted ascending with their row numbers - ties by row number - in shared memory (n <= 2048).
 __global__ void __launch_bounds__(1024)
 k_spectrum(const float *__restrict__ part, int parts, int n, int keep, float *__restrict__ S, long long *__restrict__ keep_idx, float *__restrict__ max_eig) {
+    chain_wait();
     extern __shared__ unsigned long long keys[];
     const int m = blockIdx.x;
     int size = 2;
@@ -220,6 +222,7 @@ k_spectrum(const float *__restrict__ part, int parts, int n, int keep, float *__
 __global__ void __launch_bounds__(256)
 k_row_weights(const float *__restrict__ S, const float *__restrict__ max_eig, int keep, float eps, float inv_p, float basis_bound,
               float *__restrict__ weights, float *__restrict__ bound) {
+    chain_wait();
     __shared__ float red[8];
     const int m = blockIdx.x;
     const float rho = eps >= 0.0f ? eps * max_eig[m] : 0.0f;
@@ -249,6 +252,7 @@ k_row_weights(const float *__restrict__ S, const float *__restrict__ max_eig, in
 __global__ void __launch_bounds__(256)
 k_quantize_transposed(const float *__restrict__ Q, long long ldq, long long strideQ, const float *__restrict__ code, int n, int nb,
                       float *__restrict__ absmax_base, long long stride_absmax, unsigned char *__restrict__ out_base, long long stride_out) {
+    chain_wait();
     __shared__ CodeTables<16> tab;
     __shared__ float tile[64][65];
     build_tables<16>(tab, code);
@@ -304,6 +308,7 @@ k_quantize_transposed(const float *__restrict__ Q, long long ldq, long long stri
 
 __global__ void __launch_bounds__(256)
 k_transpose(const float *__restrict__ X, long long ldx, float *__restrict__ Y, int n) {
+    chain_wait();
     __shared__ float t[32][33];
     const long long o = (long long)blockIdx.z * n * n, ox = (long long)blockIdx.z * n * ldx;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
@@ -386,7 +391,7 @@ static int to_planes(const float *X, long long ldx, long long strideX, int rows,
     return check_launch();
 }
 
-static int basis_rows(const qt_refresh_desc &d, int a, int m, const long long *index, int rows, float *X, long long ldx, const P2 &p, cudaStream_t s) {
+static int basis_rows(const qt_refresh_desc &d, int a, int m, const long long *index, int rows, float *X, long long ldx, const P2 &p, const Queue &s, bool first) {
     int shift = 0;
     while ((1 << shift) < d.blocksize) ++shift;
     const int nb = (d.n + d.blocksize - 1) / d.blocksize;
@@ -395,8 +400,8 @@ static int basis_rows(const qt_refresh_desc &d, int a, int m, const long long *i
     const dim3 grid = rows_grid((long long)rows * ((d.n + 15) / 16), m);
     const float scale = ldexpf(1.0f, kBasisExp);
     auto k = d.bits == 4 ? k_basis_rows<4> : k_basis_rows<8>;
-    k<<<grid, kThreadsR, 0, s>>>(codes, d.stride_codes, absmax, (long long)d.n * nb, d.code, d.n, nb, shift, index, d.keep, rows, X, ldx, rows * ldx,
-                                 p.hi, p.lo, p.ld, p.stride, scale);
+    if (launch_chained(k, grid, kThreadsR, 0, s, s.chained && !first, codes, d.stride_codes, absmax, (long long)d.n * nb, d.code, d.n, nb, shift, index, d.keep, rows, X, ldx, rows * ldx,
+                                 p.hi, p.lo, p.ld, p.stride, scale) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
     count_launch(1);
     return check_launch();
 }
@@ -499,7 +504,7 @@ static int refresh_pass(const qt_refresh_desc &d, int a, int m, Bump &w, bool ru
             float *v = f1, *vn = f2;
             P2 pv = p1, pn = p2, pw = p3;
             pv.exp0 = kBasisExp;
-            QT_TRY(basis_rows(d, a, m, nullptr, n, v, ld, pv, s));
+            QT_TRY(basis_rows(d, a, m, nullptr, n, v, ld, pv, s, false));
             pw.exp0 = kMaxExp - 4; pw.tmax = kMaxExp;         // entries of V V^T: at most 16
             for (int it = 0; it < d.rect_t1; ++it) {
                 Out ow; ow.P = &pw; ow.sym = 1;
@@ -511,7 +516,7 @@ static int refresh_pass(const qt_refresh_desc &d, int a, int m, Bump &w, bool ru
                 P2 tp = pv; pv = pn; pn = tp;
             }
             // L <- V_kept^T diag(S) V_kept, then w1 L + w2 G G^T (G^T G)
-            k_row_weights<<<m, 256, 0, s>>>(S, max_eig, keep, -1.0f, 0.0f, 8.0f, weights, bound);
+            if (launch_chained(k_row_weights, m, 256, 0, s, s.chained, S, max_eig, keep, -1.0f, 0.0f, 8.0f, weights, bound) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
             count_launch(1);
             P2 ra = pw, rb = pw;                              // planes of the kept rows: two halves of one buffer
             ra.ld = rb.ld = up(n, 16); ra.stride = rb.stride = keep * ra.ld;
@@ -547,16 +552,17 @@ static int refresh_pass(const qt_refresh_desc &d, int a, int m, Bump &w, bool ru
             QT_TRY(product(pl, false, pq, false, n, n, n, m, oc, s));
             int size = 2;
             while (size < n) size <<= 1;
-            k_spectrum<<<m, 1024, sizeof(unsigned long long) * size, s>>>(cd, 4 * tiles, n, keep, S, keep_idx, max_eig);
+            if (launch_chained(k_spectrum, m, 1024, sizeof(unsigned long long) * size, s, s.chained, cd, 4 * tiles, n, keep, S, keep_idx, max_eig) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
             count_launch(1);
             if (d.bits == 4 && d.blocksize == 64 && n % 16 == 0 && d.stride_codes % 8 == 0) {
                 long long ctas = (long long)nb * nb;
                 const long long cap = ((long long)device_sm_count() * 6 + m - 1) / m;      // every CTA builds the code tables
                 if (ctas > cap) ctas = cap;
-                k_quantize_transposed<<<dim3((unsigned)ctas, m), 256, 0, s>>>(Q, ld, nn, d.code, n, nb, absmax, (long long)n * nb, codes, d.stride_codes);
+                if (launch_chained(k_quantize_transposed, dim3((unsigned)ctas, m), 256, 0, s, s.chained, Q, ld, nn, d.code, n, nb, absmax, (long long)n * nb, codes,
+                                   d.stride_codes) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
                 count_launch(1);
             } else {
-                k_transpose<<<dim3((n + 31) / 32, (n + 31) / 32, m), 256, 0, s>>>(Q, ld, X, n);
+                if (launch_chained(k_transpose, dim3((n + 31) / 32, (n + 31) / 32, m), 256, 0, s, s.chained, Q, ld, X, n) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
                 count_launch(1);
                 QuantArgs qa{X, QT_F32, (long long)n * n, d.code, n, m, d.blocksize, d.bits, absmax, (long long)n * nb, nullptr, 0, codes, d.stride_codes};
                 QT_TRY(launch_quantize(qa, s));
@@ -577,7 +583,7 @@ static int refresh_pass(const qt_refresh_desc &d, int a, int m, Bump &w, bool ru
             float *r = f1, *rn = f2;
             P2 pr = p1, pn = p2;
             pr.exp0 = kBasisExp;
-            QT_TRY(basis_rows(d, a, m, keep_idx, keep, r, ld, pr, s));
+            QT_TRY(basis_rows(d, a, m, keep_idx, keep, r, ld, pr, s, !d.do_stat));
             for (int it = 0; it < d.rect_t2; ++it) {
                 Out ow; ow.P = &pw; ow.sym = 1;
                 QT_TRY(product(pr, false, pr, true, keep, keep, n, m, ow, s));
@@ -587,7 +593,7 @@ static int refresh_pass(const qt_refresh_desc &d, int a, int m, Bump &w, bool ru
                 float *tf = r; r = rn; rn = tf;
                 P2 tp = pr; pr = pn; pn = tp;
             }
-            k_row_weights<<<m, 256, 0, s>>>(S, max_eig, keep, d.eps, d.inv_p, 8.0f, weights, bound);
+            if (launch_chained(k_row_weights, m, 256, 0, s, s.chained, S, max_eig, keep, d.eps, d.inv_p, 8.0f, weights, bound) != cudaSuccess) { cudaGetLastError(); return record(QT_ERR_LAUNCH); }
             count_launch(1);
             P2 ps = pn;
             ps.exp = exps; ps.exp0 = 0; ps.tmax = kTarget;
