@@ -336,10 +336,8 @@ def op_ema_gram(L, G, axis, w1, w2):
 def op_ema_gram_selected(L, sel, G, axis, w1, w2):
     """op_ema_gram on the matrices L[sel[k]] with G[k], updated in place: the product reads its C
     operand and writes its result through the slot list, so the selected matrices are neither
-    gathered into a temporary nor scattered back (sel: int32 device tensor).  Where products have to be
-    exact (_EXACT) the operands are three bf16 planes, 24 bits, instead of an fp32 library product on the
-    SIMT units.  All tiles are computed: L comes from row-blocked 4-bit state and is not quite symmetric."""
-    P = Mat(G).planes if _tc(L) else Mat(G).planes3
+    gathered into a temporary nor scattered back (sel: int32 device tensor)."""
+    P = Mat(G).planes
     _gemm.gemm_ex(P, P, trans_a=(axis == 1), trans_b=(axis == 0), alpha=w2, beta=w1, C=L, D=L,
                   d_slot=sel, c_follows_d=True, batch=G.shape[0])
     return L
@@ -434,11 +432,10 @@ def _ema_update(L, grads_axes, w1, w2):
         groups[(tuple(g.shape), axis)].append(k)
     for (shape, axis), ks in groups.items():
         Gs = torch.stack([grads_axes[k][0].float() for k in ks])
-        # orders below a tile's smallest useful size keep the library product in exact mode
-        if USE_TENSOR_CORES and L.is_cuda and F.lib is not None and L.is_contiguous() and (not _EXACT or L.shape[1] >= 64):
-            L = op_ema_gram_selected(L, _index_tensor(ks, L.device, torch.int32), Gs, axis, w1, w2)
-        elif len(ks) == L.shape[0]:
+        if len(ks) == L.shape[0]:
             L = op_ema_gram(L, Gs, axis, w1, w2)
+        elif _tc(L) and L.is_contiguous():
+            L = op_ema_gram_selected(L, _index_tensor(ks, L.device, torch.int32), Gs, axis, w1, w2)
         else:
             sel = _index_tensor(ks, L.device)
             L[sel] = op_ema_gram(L[sel], Gs, axis, w1, w2)
